@@ -3,8 +3,8 @@
 // Fused path (tn_march_count + tn_march_emit): no host round trip, one sequential march.
 //  * count: one thread per ray runs the reference's DDA loop with its exact arithmetic, written
 //    branch-free per step (both successors of t are computed, one is selected) so that a warp's
-//    rays never split. Shared memory holds a Morton spread table and a coarse occupancy mip
-//    that answers empty 4x4x4 blocks without a global load. A box holding every occupied cell
+//    rays never split. Shared memory holds a coarse occupancy mip that answers empty 4x4x4
+//    blocks without a global load; the loads of the others are checked a few steps later. A box holding every occupied cell
 //    ends each ray's loop where it leaves that box for good (the count cannot change after).
 //    The t of every occupied step goes to a per-ray slot. Each 64-ray block reduces its counts;
 //    the last block to finish (ticket) scans the block totals and performs the reference's
@@ -331,15 +331,32 @@ __device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) 
 // level 0's times 2^k (2^-k): scaling by a power of two is exact in IEEE arithmetic, and the
 // host checks every level against the per-level table before launching.
 struct CountGrid {
-    float cell0, inv_ls0, res_f;
+    float cell0;
+    float half_res;              // R / 2
     int half0_bits, cell0_bits;  // bit patterns of the level-0 half extent and cell size
+    int half0_below, cell0_below;  // those of half of them: one less in the exponent
+    int scale0_bits;             // bit pattern of R / level-0 size
     uint32_t res_m1;             // R - 1
     int res_shift;               // log2 R
-    uint32_t plane_words;        // R^3 / 32: words per level of the bit-planes
-    int n_levels;
-    const uint8_t* __restrict__ bits;     // the bitfield, one byte per cell (bit k = level k)
-    const uint32_t* __restrict__ planes;  // the same bits as one plane per level, 32 cells per word
+    int level_max;               // number of levels - 1
+    float res_below;             // the float below R
+    int mode;                    // CountMode
+    const uint8_t* __restrict__ bits;  // the bitfield, one byte per cell (bit k = level k)
+    // the same bits as two planes per level, [level][2][blocks]: cell (x, y, z) of a 4x4x4 block at
+    // plane z >> 1, bit 31 - (16 (z & 1) + 4 y + x); blocks x-fastest as the coarse mip
+    const uint32_t* __restrict__ planes;
+    float inv_dt_lo;             // 1 / dt_min - inv_dt_min, rounded
 };
+
+// Forms of the count loop, picked on the host from the grid and the box (make_count_grid):
+//  BYTES    no coarse mip (R < 16 or R > 128): the bitfield byte of every step is read;
+//  MIP      coarse mip and bit-planes, any geometry;
+//  BOUNDED  and the box lies inside the coarsest level, so that every scaled cell coordinate is in
+//           [0, R] (a size times its rounded reciprocal rounds to at most 1) and floor is one
+//           round-down addition: no conversion instructions;
+//  POW2     and the level sizes are powers of two, so that x times the level's scale is exact and
+//           the scaled coordinate is one fused multiply-add.
+enum CountMode : int { COUNT_BYTES = 0, COUNT_MIP = 1, COUNT_BOUNDED = 2, COUNT_POW2 = 3 };
 
 // get_grid_level_at (occupancy-grid.cuh:232-248): the finest level whose extent holds the point
 // (max |coordinate| m < half extent) and whose cell is larger than dt, else the coarsest. Each
@@ -349,56 +366,32 @@ struct CountGrid {
 //   m < half0 * 2^j  <=>  j > (bits(m) - bits(half0)) / 2^23,
 //   cell0 * 2^j > dt  <=>  j > (bits(dt) - bits(cell0)) / 2^23,
 // and the first such j is the quotient (an arithmetic shift) plus one, at least 0.
-// NL = 0: the level count is only known at run time (nl_rt).
-template <int NL>
-__device__ __forceinline__ int count_level(float m, float dt, int half0_bits, int cell0_bits, int nl_rt) {
-    const int jp = (__float_as_int(m) - half0_bits) >> 23;
-    const int jd = (__float_as_int(dt) - cell0_bits) >> 23;
-    return min(max(max(jp, jd) + 1, 0), (NL ? NL : nl_rt) - 1);
+__device__ __forceinline__ int level_of(int half0_below, int cell0_below, int level_max, float m, float dt) {
+    const int d = max(__float_as_int(m) - half0_below, __float_as_int(dt) - cell0_below);
+    return min(max(d >> 23, 0), level_max);
 }
 
-// a / b rounded toward +infinity for finite a >= b > 0 (the __fdiv_ru of get_dt_to_next_voxel,
-// occupancy-grid.cuh:281), from inv_b = 1/b rounded to nearest. q0 = a * inv_b is within two
-// ulps of a/b; one Newton correction with the residual a - q0*b (Markstein's division
-// refinement) puts q within half an ulp plus a negligible term. RU(a/b) is the smallest float q
-// with q*b >= a, so it is q, q's successor or q's predecessor; a fused multiply-add gives the
-// residual a - q*b with the sign of the exact residual (no underflow for these operands), which
-// decides between them. (An infinite a, which only a direction of three zero components can
-// produce, yields NaN instead of infinity; either one ends the march loop the same way.)
-__device__ __forceinline__ float div_ru_pos(float a, float b, float inv_b) {
-    const float q0 = __fmul_rn(a, inv_b);
-    float q = __fmaf_rn(__fmaf_rn(-q0, b, a), inv_b, q0);
-    if (__fmaf_rn(-q, b, a) > 0.0f) {
-        q = __uint_as_float(__float_as_uint(q) + 1u);
-    } else {
-        const float d = __uint_as_float(__float_as_uint(q) - 1u);
-        if (__fmaf_rn(-d, b, a) <= 0.0f) q = d;
-    }
-    return q;
-}
-
-// One axis of get_dt_to_next_voxel (occupancy-grid.cuh:270-278) from the scaled coordinate
-// f = (p / level size + 0.5) * R, which is also the cell coordinate before truncation.
-__device__ __forceinline__ float axis_dt(float f, float h, float inv_d, float kcell) {
-    return __fmul_rn(kcell, __fmul_rn(__fadd_rn(floorf(__fadd_rn(__fadd_rn(h, f), 0.5f)), -f), inv_d));
+// One axis of get_dt_to_next_voxel (occupancy-grid.cuh:270-278), before its factor cell size, from
+// the scaled coordinate f = (p / level size + 0.5) * R, which is also the cell coordinate before
+// truncation. FAST: f in [0, R], where adding 1.5 * 2^23 with rounding down leaves floor + 1.5 * 2^23.
+template <bool FAST>
+__device__ __forceinline__ float axis_cells(float f, float h, float inv_d) {
+    const float v = __fadd_rn(__fadd_rn(h, f), 0.5f);
+    const float fl = FAST ? __fadd_rn(__fadd_rd(v, 12582912.0f), -12582912.0f) : floorf(v);
+    return __fmul_rn(__fadd_rn(fl, -f), inv_d);
 }
 
 // Cell coordinate of get_voxel_morton_index, clamped to the grid: the conversion saturates
 // (negative and NaN give 0), then the upper edge clamps to R - 1.
 __device__ __forceinline__ uint32_t cell_of(float f, uint32_t res_m1) { return min(__float2uint_rz(f), res_m1); }
 
-// The march loop of march_and_count_steps_per_ray_kernel (training-batch-kernels.cuh:258-297),
-// branch-free per step so that the 32 rays of a warp never split: both successors of t (the
-// occupied step t + dt and the DDA skip) are computed and one is selected. The scaled cell
-// coordinates are computed once per step and shared by the Morton lookup and the skip (the
-// reference computes the same expression in both, occupancy-grid.cuh:155-159 and :268-272).
-//  * t_lim = min(the float below t_max, t_stop) merges `t < t_max` with the tail cut: past
-//    t_stop the ray stays outside every occupied cell, so the loop ends with the same count.
-//  * the box test (`if (!bbox.contains(p)) break`, training-batch-kernels.cuh:263-265) is made
-//    once at the first step and folded into t_lim for the others (box_exit_t below).
-//  * LIMIT: max_steps (otherwise unlimited) ends the ray after that many occupied steps.
-//  * spread holds three Morton spread tables, pre-shifted for x, y and z.
-//  * slots record the t of the first slot_cap occupied steps for the emit pass.
+// The same in the low bits of the result. FAST (f in [0, R]): f + 2^23 rounded down holds the
+// cell in its mantissa.
+template <bool FAST>
+__device__ __forceinline__ uint32_t cell_bits(float res_below, uint32_t res_m1, float f) {
+    return FAST ? __float_as_uint(__fadd_rd(fminf(f, res_below), 8388608.0f)) : cell_of(f, res_m1);
+}
+
 // Order-preserving map of the non-NaN floats to unsigned integers (a < b <=> key(a) < key(b)).
 __device__ __forceinline__ uint32_t float_key(float f) {
     const uint32_t b = __float_as_uint(f);
@@ -434,90 +427,214 @@ __device__ __forceinline__ float box_exit_t(const tn_bbox& b, const RayMarch& r,
                  fminf(axis_exit_t(r.oy, r.dy, b.min_y, b.max_y, t0), axis_exit_t(r.oz, r.dz, b.min_z, b.max_z, t0)));
 }
 
-template <int NL, bool MIP, bool LIMIT>
+// The march loop of march_and_count_steps_per_ray_kernel (training-batch-kernels.cuh:258-297). A
+// ray's steps form one dependent chain, and a batch holds about one warp per scheduler, so the
+// kernel takes as long as the longest chain: what counts is the latency from t to the next t.
+//  * Branch-free step: both successors of t (the occupied step t + dt and the DDA skip) are
+//    computed and one is selected, so that the 32 rays of a warp never split.
+//  * The occupancy lookup is off the chain. A step goes on with a guess (its cell is what the last
+//    checked cell was) while its bit-plane word is on the way, and is checked D steps later; the
+//    coarse mip in shared memory spares the words of empty 4x4x4 blocks. A wrong guess puts t, n and the iteration count back to that step, which then
+//    runs again with the right guess, and drops the steps made since. Rays cross occupied space in
+//    runs, so a guess fails a few times per surface. Words travel through shared memory (cp.async,
+//    one group a step).
+//  * Selects on the chain are bitwise with masks: a predicate costs about three such operations.
+//  * The cell lookup and the skip run at the level of the previous step (k) while the step's own
+//    level is found beside them; where the two differ (a ray changes level a handful of times) the
+//    step is discarded without moving and runs again at the new level.
+//  * f = (p / size + 0.5) * R is evaluated as p * (R / size) + R / 2: R is a power of two, so both
+//    roundings scale. The factor cell size of the three axis distances is applied after their
+//    minimum (rounding is monotone).
+//  * t_skip: t_target / dt_min rounded up, times dt_min. With 1 / dt_min as an unevaluated sum of
+//    two floats (inv_dt_min + inv_dt_lo, relative error below 2^-48), q = t_target * that is off
+//    a / b by less than 2^-47 relatively before its one rounding, and a / b is either a float or at
+//    least 2^-48 away from one, so q is one of the two floats around a / b (a / b itself when it is
+//    one). The fused residual a - q b has the sign of the exact one (dt_min >= 1e-30: no
+//    underflow); when it is positive q lies below a / b and its successor is the quotient rounded
+//    up. (An infinite t_target, which only a direction of three zero components can produce, gives
+//    NaN instead of infinity; either one ends the loop.)
+//  * t_lim = min(the float below t_max, t_stop, box exit) merges `t < t_max`, the tail cut (past
+//    t_stop the ray stays outside every occupied cell) and the box test
+//    (training-batch-kernels.cuh:263-265; box_exit_t above).
+//  * slots record the t of the first slot_cap occupied steps for the emit pass; a step that a wrong
+//    guess recorded is overwritten, or lies past the final count.
+// Bound: issue and dependent latency of one warp a scheduler, about 100 instructions and 190 cycles
+// a step (600 with the lookup on the chain). The kernel alone on B200: 2^14 rays through 5 cascades
+// of 128^3 164 -> 77 us, 256 rays of 1024 samples through one cascade 314 -> 121 us, sixteen scenes
+// of 2.5e5 rays (persistent launch, many warps a scheduler) 1238 -> 730 us. Depths measured on
+// the first two: 3 84 and 158 us, 4 83 and 140, 5 78 and 134, 6 76 and 129, 8 78 and 118; on the
+// scenes 3 is the best. Words kept in registers instead of shared memory cost 10% (the loads then
+// share the few scoreboards and wait for each other).
+constexpr int COUNT_DEPTH = 6;        // steps in flight, one launch a batch
+constexpr int COUNT_RING = 4 * (COUNT_DEPTH | 1);  // bytes a thread of shared memory (an odd number of words: no bank conflicts)
+constexpr int COUNT_DEPTH_MULTI = 3;  // of the persistent launch, which has warps to hide the lookups behind
+
+// Copies the word at p into shared memory asynchronously, or zero when `bytes` is 0 instead of 4.
+__device__ __forceinline__ void fetch_word(uint32_t dst, const uint32_t* p, uint32_t bytes) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(p), "r"(bytes));
+}
+__device__ __forceinline__ float in_reg(float v) {
+    asm volatile("" : "+f"(v));
+    return v;
+}
+__device__ __forceinline__ int in_reg(int v) {
+    asm volatile("" : "+r"(v));
+    return v;
+}
+// a where the mask is all ones, b where it is zero.
+__device__ __forceinline__ float pick(uint32_t mask, float a, float b) {
+    return __uint_as_float((__float_as_uint(a) & mask) | (__float_as_uint(b) & ~mask));
+}
+__device__ __forceinline__ void fetch_commit() { asm volatile("cp.async.commit_group;"); }
+template <int N>
+__device__ __forceinline__ void fetch_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N)); }
+__device__ __forceinline__ uint32_t read_word(uint32_t src) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(src));
+    return v;
+}
+__device__ __forceinline__ void store_if(bool on, float* p, float v) {
+    asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.global.f32 [%1], %2; }" ::"r"((uint32_t)on), "l"(p), "f"(v));
+}
+
+// GUARD: the iteration limit can be reached (count_ray); without it the loop needs no count of
+// its iterations.
+template <int MODE, int D, bool GUARD>
 __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, const RayMarch& r, float t_lim,
                                    uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
-                                   const uint32_t* __restrict__ spread, float* __restrict__ slots,
+                                   const uint32_t* __restrict__ spread, uint32_t ring, float* __restrict__ slots,
                                    uint32_t slot_cap) {
+    constexpr bool MIP = MODE != COUNT_BYTES;
+    constexpr bool FAST = MODE >= COUNT_BOUNDED;
     const float hx = __fmul_rn(0.5f, copysignf(1.0f, r.dx));
     const float hy = __fmul_rn(0.5f, copysignf(1.0f, r.dy));
     const float hz = __fmul_rn(0.5f, copysignf(1.0f, r.dz));
-    const int cs = cg.res_shift - 2;
-    const uint32_t res = 1u << cg.res_shift;
-    uint32_t n = 0, iters = 0;
+    const uint32_t C = 1u << (cg.res_shift - 2), C3 = C * C * C, res = 1u << cg.res_shift;
+    const uint32_t max_iters = a.max_iters;
+    // the loop's constants in registers: read from the parameters they would be loaded again each trip
+    const float cone = in_reg(a.cone), dt_min = in_reg(a.dt_min), dt_max = in_reg(a.dt_max);
+    const float inv_dt = in_reg(a.inv_dt_min), inv_dt_lo = in_reg(cg.inv_dt_lo), half_res = in_reg(cg.half_res);
+    const float res_below = in_reg(cg.res_below);
+    const int scale0 = in_reg(cg.scale0_bits), cell0 = in_reg(cg.cell0_bits);
+    const int half_below = in_reg(cg.half0_below), cell_below = in_reg(cg.cell0_below), kmax = in_reg(cg.level_max);
+    uint32_t n = 0, iters = 0, guess = 0;  // guess: all ones (occupied) or zero
     float t = r.t;
-    // Level prediction: the cell lookup and the DDA skip of an iteration run at the level of the
-    // previous iteration (kp), while the iteration's own level is found beside them; when the two
-    // differ (a ray changes level a handful of times) the iteration is discarded without moving
-    // and runs again at the new level. The level choice is then off the chain from t to the next
-    // t, and every iteration that counts used the level the reference's loop uses.
-    int kp;
+    int k;
     {
         float x, y, z;
         ray_point(r, t, x, y, z);
-        const float m = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
-        kp = count_level<NL>(m, get_dt(t, a.cone, a.dt_min, a.dt_max), cg.half0_bits, cg.cell0_bits, cg.n_levels);
+        k = level_of(half_below, cell_below, kmax, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))), get_dt(t, cone, dt_min, dt_max));
     }
-    float ils = __fmul_rn(cg.inv_ls0, pow2i(-kp)), kc = __fmul_rn(cg.cell0, pow2i(kp));
-    // the iteration guard is part of the loop condition (no branch with a side effect in the
-    // body, which stays one straight block); the flag is raised after the loop
-    const uint32_t max_iters = a.max_iters;
-    while ((t <= t_lim) & (iters < max_iters)) {
-        float x, y, z;
-        ray_point(r, t, x, y, z);
-        const float dt = get_dt(t, a.cone, a.dt_min, a.dt_max);
-        const float m = fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z)));
-        const int k = count_level<NL>(m, dt, cg.half0_bits, cg.cell0_bits, cg.n_levels);
-        const bool same_level = k == kp;
-        const float fx = __fmul_rn(__fadd_rn(__fmul_rn(x, ils), 0.5f), cg.res_f);
-        const float fy = __fmul_rn(__fadd_rn(__fmul_rn(y, ils), 0.5f), cg.res_f);
-        const float fz = __fmul_rn(__fadd_rn(__fmul_rn(z, ils), 0.5f), cg.res_f);
-        const uint32_t cx = cell_of(fx, cg.res_m1), cy = cell_of(fy, cg.res_m1), cz = cell_of(fz, cg.res_m1);
-        const uint32_t idx = spread[cx] | spread[res + cy] | spread[2 * res + cz];
-        bool occ;
-        if (MIP) {
-            const uint32_t coarse = mip[(((((cz >> 2) << cs) | (cy >> 2)) << cs) | (cx >> 2))];
-            const uint32_t word = ((coarse >> kp) & 1u) ? __ldg(cg.planes + kp * cg.plane_words + (idx >> 5)) : 0u;
-            occ = (word >> (idx & 31u)) & 1u;
-        } else {
-            occ = (__ldg(cg.bits + idx) >> kp) & 1u;
+    // steps in flight: the word read (in shared memory; `word`: of the next check), its left shift
+    // that brings the cell's bit to the sign, whether there is anything to check (all ones), and
+    // t, n, iters before the step
+    uint32_t word = 0, bit[D], check[D], n0[D], it0[D];
+    float t0[D];
+#pragma unroll
+    for (int j = 0; j < D; ++j) bit[j] = check[j] = n0[j] = it0[j] = 0u, t0[j] = 0.0f;
+#pragma unroll
+    for (int j = 0; j < D - 1; ++j) fetch_commit();
+    // a bound that no ray reaches (a step is made at most D + 1 times, level changes apart)
+    uint32_t trips = max_iters < 0x7FFFFF00u ? 2u * max_iters + 64u : 0xFFFFFFFFu;
+    for (;;) {
+#pragma unroll
+        for (int j = 0; j < D; ++j) {
+            // Check the step made D steps ago. The steps in flight were all made under the current
+            // guess; a wrong one goes back to it, turns the guess and drops the steps since.
+            const uint32_t truth = (uint32_t)((int)__funnelshift_l(0u, word, bit[j]) >> 31);
+            const uint32_t wrong = (truth ^ guess) & check[j];
+            fetch_wait<D - 2>();
+            word = read_word(ring + ((j + 1) % D) * 4);
+            t = pick(wrong, t0[j], t);
+            n = (n0[j] & wrong) | (n & ~wrong);
+            if (GUARD) iters = (it0[j] & wrong) | (iters & ~wrong);
+            guess ^= wrong;
+#pragma unroll
+            for (int i = 1; i < D; ++i) check[(j + i) % D] &= ~wrong;
+            // one step
+            float x, y, z;
+            ray_point(r, t, x, y, z);
+            // get_dt: the clamp of a number (t is one in a live step)
+            const float dt = fminf(fmaxf(__fmul_rn(t, cone), dt_min), dt_max);
+            const int kn = level_of(half_below, cell_below, kmax, fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))), dt);
+            const bool live = (t <= t_lim) & (n < max_steps) & (!GUARD || iters < max_iters);
+            const uint32_t go = live & (kn == k) ? ~0u : 0u;
+            const float s = __int_as_float(scale0 - (k << 23)), kc = __int_as_float(cell0 + (k << 23));
+            float fx, fy, fz;
+            if (MODE == COUNT_POW2) {
+                fx = __fmaf_rn(x, s, half_res);
+                fy = __fmaf_rn(y, s, half_res);
+                fz = __fmaf_rn(z, s, half_res);
+            } else {
+                fx = __fadd_rn(__fmul_rn(x, s), half_res);
+                fy = __fadd_rn(__fmul_rn(y, s), half_res);
+                fz = __fadd_rn(__fmul_rn(z, s), half_res);
+            }
+            const uint32_t cx = cell_bits<FAST>(res_below, cg.res_m1, fx), cy = cell_bits<FAST>(res_below, cg.res_m1, fy), cz = cell_bits<FAST>(res_below, cg.res_m1, fz);
+            if (MIP) {
+                // the mask drops what lies above the cells' bits, and keeps a lane past its end in the table
+                const uint32_t blk = (((cz >> 2) * C + (cy >> 2)) * C + (cx >> 2)) & (C3 - 1u);
+                fetch_word(ring + j * 4,
+                           cg.planes + ((uint32_t)k * (2u * C3) + (cz & 2u) * (C3 >> 1) + blk),
+                           ((uint32_t)mip[blk] >> k << 2) & 4u);
+                bit[j] = (cz << 4 & ~15u) | (((cy << 2 & 12u) | (cx & ~12u)) & 15u);  // taken modulo 32
+            } else {
+                const uint32_t idx = spread[cx] | spread[res + cy] | spread[2 * res + cz];
+                fetch_word(ring + j * 4, reinterpret_cast<const uint32_t*>(cg.bits) + (idx >> 2), 4u);
+                bit[j] = 31u - (idx & 3u) * 8u - (uint32_t)k;
+            }
+            fetch_commit();
+            const float gap = fminf(fminf(axis_cells<FAST>(fx, hx, r.idx), axis_cells<FAST>(fy, hy, r.idy)),
+                                    axis_cells<FAST>(fz, hz, r.idz));
+            const float t_target = fmaxf(dt_min, __fmul_rn(kc, gap));
+            const float q = __fmaf_rn(t_target, inv_dt, __fmul_rn(t_target, inv_dt_lo));
+            const float over = __fmaf_rn(q, dt_min, -t_target);  // negative: q lies below the quotient
+            const float qu = __uint_as_float(__float_as_uint(q) + (__float_as_uint(over) >> 31));
+            const float skip = __fmul_rn(qu, dt_min);
+            check[j] = go;
+            t0[j] = t;
+            n0[j] = n;
+            if (GUARD) it0[j] = iters;
+            const uint32_t occ = go & guess;
+            store_if((occ != 0u) & (n < slot_cap), slots + n, t);
+            // t + dt, t + skip, or t + 0
+            t = __fadd_rn(t, __uint_as_float((__float_as_uint(dt) & occ) | (__float_as_uint(skip) & (go & ~guess))));
+            n -= occ;
+            if (GUARD) iters -= go;
+            k = kn;
         }
-        // DDA skip to the next cell boundary: t_target / dt_min rounded up (to a float), times dt_min
-        const float tx = axis_dt(fx, hx, r.idx, kc);
-        const float ty = axis_dt(fy, hy, r.idy, kc);
-        const float tz = axis_dt(fz, hz, r.idz, kc);
-        const float t_target = fmaxf(a.dt_min, fminf(fminf(tx, ty), tz));
-        const float t_skip = __fadd_rn(t, __fmul_rn(div_ru_pos(t_target, a.dt_min, a.inv_dt_min), a.dt_min));
-        // branch-free step: the slot store runs every iteration (a skip's t is overwritten by the
-        // next occupied step, and the emit pass reads only the first n slots), so the select of
-        // the successor carries no branch
-        if (n < slot_cap) slots[n] = t;
-        const float t_occ = __fadd_rn(t, dt);
-        const float t_next = occ ? t_occ : t_skip;
-        t = same_level ? t_next : t;
-        n += (same_level & occ) ? 1u : 0u;
-        iters += same_level ? 1u : 0u;
-        kp = k;
-        ils = __fmul_rn(cg.inv_ls0, pow2i(-k));
-        kc = __fmul_rn(cg.cell0, pow2i(k));
-        if (LIMIT && n >= max_steps) break;
+        // nothing in flight and nothing left
+        uint32_t pending = 0;
+#pragma unroll
+        for (int j = 0; j < D; ++j) pending |= check[j];
+        --trips;
+        if ((!pending & !((t <= t_lim) & (n < max_steps) & (!GUARD || iters < max_iters))) | (trips == 0u)) break;
     }
-    if (iters >= max_iters && t <= t_lim && !(LIMIT && n >= max_steps)) raise_flag(flags, ERR_GUARD);
+    if (trips == 0u || (GUARD && iters >= max_iters && t <= t_lim && n < max_steps)) raise_flag(flags, ERR_GUARD);
     return n;
 }
 
-template <int NL, bool MIP>
-__device__ uint32_t count_ray(const MarchArgs& a, const CountGrid& cg, const RayMarch& r, float t_lim,
-                              uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
-                              const uint32_t* __restrict__ spread, float* __restrict__ slots, uint32_t slot_cap) {
+template <int MODE, int D>
+__device__ __forceinline__ uint32_t count_ray(const MarchArgs& a, const CountGrid& cg, const RayMarch& r, float t_lim,
+                                              uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
+                                              const uint32_t* __restrict__ spread, uint32_t ring,
+                                              float* __restrict__ slots, uint32_t slot_cap) {
     if (!(r.t <= t_lim)) return 0;  // no step (a NaN limit included)
     float x, y, z;
     ray_point(r, r.t, x, y, z);
     if (!bbox_contains(a.bbox, x, y, z)) return 0;  // the first step leaves the box
     t_lim = fminf(t_lim, box_exit_t(a.bbox, r, r.t));
-    return max_steps == 0xffffffffu
-               ? count_ray_loop<NL, MIP, false>(a, cg, r, t_lim, max_steps, flags, mip, spread, slots, slot_cap)
-               : count_ray_loop<NL, MIP, true>(a, cg, r, t_lim, max_steps, flags, mip, spread, slots, slot_cap);
+    if (MODE >= COUNT_BOUNDED) {
+        // Every step moves t by at least dt_min before rounding. Where dt_min is at least four
+        // spacings of the floats up to t_lim, that leaves 7/8 dt_min, which bounds the iterations.
+        const float far = fmaxf(fabsf(r.t), fabsf(t_lim));
+        const bool safe = a.dt_min >= far * 4.8e-7f && fminf(fminf(fabsf(r.idx), fabsf(r.idy)), fabsf(r.idz)) < 1e30f &&
+                          (t_lim - r.t) < 0.8f * a.dt_min * (float)(a.max_iters >> 1);
+        if (safe)
+            return count_ray_loop<MODE, D, false>(a, cg, r, t_lim, max_steps, flags, mip, spread, ring, slots, slot_cap);
+    }
+    return count_ray_loop<MODE == COUNT_BYTES ? COUNT_BYTES : COUNT_MIP, D, true>(a, cg, r, t_lim, max_steps, flags,
+                                                                                  mip, spread, ring, slots, slot_cap);
 }
 
 // World-space box that holds every occupied cell of every level: per level, the box of its
@@ -534,8 +651,8 @@ __device__ void occupied_union(const CountGrid& cg, const int* __restrict__ box,
         const float ls = __int_as_float(cg.half0_bits) * pow2i(k + 1), cw = cg.cell0 * pow2i(k);
         for (int ax = 0; ax < 3; ++ax) {
             const int l = box[k * 3 + ax], h = box[MAX_LEVELS * 3 + k * 3 + ax];
-            float wl = (4.0f * (float)l / cg.res_f - 0.5f) * ls - cw;
-            float wh = (4.0f * (float)h / cg.res_f - 0.5f) * ls + cw;
+            float wl = (4.0f * (float)l / (2.0f * cg.half_res) - 0.5f) * ls - cw;
+            float wh = (4.0f * (float)h / (2.0f * cg.half_res) - 0.5f) * ls + cw;
             if (k == n_levels - 1) {
                 if (l == 0) wl = -INFINITY;
                 if (h == C) wh = INFINITY;
@@ -577,11 +694,11 @@ __device__ __forceinline__ bool ray_box_exit(const RayMarch& r, const float* u, 
     return true;
 }
 
-// One thread per ray, blockDim.x rays per block (a tuning choice, 32..256). Shared memory: the three Morton spread tables
-// (3 R words) and, with MIP, the coarse mip (R^3/64 bytes); with MIP the fine test reads the
-// per-level bit-planes. The last block to finish scans the group totals and applies the batch
+// One thread per ray, blockDim.x rays per block (a tuning choice, 32..256). Shared memory: the coarse
+// mip (R^3/64 bytes; the fine test reads the per-level bit-planes), or without it the three Morton
+// spread tables (3 R words). The last block to finish scans the group totals and applies the batch
 // cut on the device.
-template <int NL, bool MIP>
+template <int MODE>
 __global__ void __launch_bounds__(COUNT_GROUP_MAX)
 march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* __restrict__ n_rays_dev, uint32_t rs,
                    const float* __restrict__ ori, const float* __restrict__ dir, const float* __restrict__ ray_t,
@@ -589,19 +706,24 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
                    uint32_t batch_size, uint32_t* batch_info, uint32_t* block_agg, uint32_t* block_prefix,
                    uint32_t* ticket, uint32_t* flags, const uint8_t* __restrict__ mip_g,
                    const int* __restrict__ box_g, float* __restrict__ slots, uint32_t slot_cap) {
+    constexpr bool MIP = MODE != COUNT_BYTES;
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* spread = reinterpret_cast<uint32_t*>(smem);
-    uint8_t* mip = smem + ((size_t)12 << cg.res_shift);
+    uint8_t* mip = smem;
+    // after the tables: the words of the steps in flight, COUNT_DEPTH a thread
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(
+        smem + (MIP ? (size_t)1 << (3 * (cg.res_shift - 2)) : (size_t)12 << cg.res_shift) + COUNT_RING * threadIdx.x);
     __shared__ float ubox_s[6];
     __shared__ int cut_s;
-    const uint32_t res = 1u << cg.res_shift;
-    for (uint32_t c = threadIdx.x; c < res; c += blockDim.x) {
-        const uint32_t v = part1by2(c);
-        spread[c] = v;
-        spread[res + c] = v << 1;
-        spread[2 * res + c] = v << 2;
-    }
-    if (MIP) {
+    if (!MIP) {
+        const uint32_t res = 1u << cg.res_shift;
+        for (uint32_t c = threadIdx.x; c < res; c += blockDim.x) {
+            const uint32_t v = part1by2(c);
+            spread[c] = v;
+            spread[res + c] = v << 1;
+            spread[2 * res + c] = v << 2;
+        }
+    } else {
         const uint32_t n16 = (1u << (3 * (cg.res_shift - 2))) / 16;
         const uint4* src = reinterpret_cast<const uint4*>(mip_g);
         uint4* dst = reinterpret_cast<uint4*>(mip);
@@ -629,9 +751,8 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
             const float below = nextafterf(t_max, -INFINITY);
             const float t_lim = t_stop < below ? t_stop : below;  // a NaN t_max stays NaN
             if (meets)
-                cnt = count_ray<NL, MIP>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip,
-                                         spread, slots ? slots + (size_t)i * slot_cap : nullptr,
-                                         slots ? slot_cap : 0u);
+                cnt = count_ray<MODE, COUNT_DEPTH>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip, spread, ring,
+                                      slots ? slots + (size_t)i * slot_cap : nullptr, slots ? slot_cap : 0u);
             if (cnt == 0) alive[i] = 0;
         }
         counts[i] = cnt;
@@ -731,22 +852,23 @@ expand_kernel(MarchArgs a, float inv_aabb, uint32_t n_rays, const uint32_t* __re
     expand_ray(a, inv_aabb, r_i, o0, n, rs, img_id, ori, dir, ray_t, o, slots, slot_cap, sub, L);
 }
 
-// Bits k of the four bytes of x (cells 4j .. 4j+3) as four consecutive bits: the mask leaves
-// them at bit positions 0, 8, 16, 24, and the multiply by 1 + 2^7 + 2^14 + 2^21 moves them to
-// 21..24 without any two partial products meeting.
+// Bits k of the four bytes of x, Morton cells 4j .. 4j+3 (x0 y0 = 00, 10, 01, 11), at the bits 0, 1,
+// 4, 5 of a block's linear cell order: the mask leaves them at positions 0, 8, 16, 24, and the
+// multiply by 2^24 + 2^17 + 2^12 + 2^5 moves them to 24, 25, 28, 29 (every other partial product
+// falls below 24 or out of the word, at positions of its own).
 __device__ __forceinline__ uint32_t gather_level_bits(uint32_t x, int k) {
-    return ((((x >> k) & 0x01010101u) * 0x00204081u) >> 21) & 0xFu;
+    return ((((x >> k) & 0x01010101u) * 0x01021020u) >> 24) & 0x33u;
 }
 
 // Coarse occupancy mip, x-fastest: byte (cz*C + cy)*C + cx (C = R/4) is the OR of the 64 fine
 // bytes of that 4x4x4 block, Morton indices [64m, 64m + 64) with m = morton(cx, cy, cz). Also
-//  * writes the per-level bit-planes: bit j of word w of plane k is bit k of cell 32w + j
-//    (words 2m and 2m + 1 of every plane come from this block);
+//  * writes the per-level bit-planes: bit k of this block's cells, cell (x, y, z) of the block in
+//    plane 2k + (z >> 1) at bit 31 - (16 (z & 1) + 4 y + x);
 //  * reduces, per level, the box of occupied blocks into box[lo x,y,z per level | hi+1 x,y,z
 //    per level] (lo starts at a large value, hi at 0), the input of the count pass's tail cut.
 __device__ __forceinline__ void build_mip_block(int cshift, int n_levels, const uint4* __restrict__ bits,
-                                                uint8_t* __restrict__ mip, int* box, uint32_t* __restrict__ planes,
-                                                uint32_t plane_words, uint32_t block) {
+                                                uint8_t* __restrict__ mip, int* box,
+                                                uint32_t* __restrict__ planes, uint32_t block) {
     __shared__ int sbox[BOX_INTS];
     if (threadIdx.x < BOX_INTS) sbox[threadIdx.x] = threadIdx.x < BOX_INTS / 2 ? 0x7fffffff : 0;
     __syncthreads();
@@ -772,12 +894,14 @@ __device__ __forceinline__ void build_mip_block(int cshift, int n_levels, const 
             uint32_t lo = 0, hi = 0;
             if ((v >> k) & 1u) {
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
-                    lo |= gather_level_bits(w[j], k) << (4 * j);
-                    hi |= gather_level_bits(w[8 + j], k) << (4 * j);
+                for (int j = 0; j < 8; ++j) {  // bits of j: z0, x1, y1 (z1 picks the word)
+                    const int at = 16 * (j & 1) + 2 * ((j >> 1) & 1) + 8 * (j >> 2);
+                    lo |= gather_level_bits(w[j], k) << at;
+                    hi |= gather_level_bits(w[8 + j], k) << at;
                 }
             }
-            *reinterpret_cast<uint2*>(planes + (size_t)k * plane_words + 2 * (size_t)m) = make_uint2(lo, hi);
+            planes[((size_t)(2 * k) << (3 * cshift)) + c] = __brev(lo);
+            planes[((size_t)(2 * k + 1) << (3 * cshift)) + c] = __brev(hi);
         }
     }
     for (int k = 0; k < n_levels; ++k) {
@@ -811,8 +935,8 @@ __device__ __forceinline__ void build_mip_block(int cshift, int n_levels, const 
 
 __global__ void __launch_bounds__(256)
 build_mip_kernel(int cshift, int n_levels, const uint4* __restrict__ bits, uint8_t* __restrict__ mip, int* box,
-                 uint32_t* __restrict__ planes, uint32_t plane_words) {
-    build_mip_block(cshift, n_levels, bits, mip, box, planes, plane_words, blockIdx.x);
+                 uint32_t* __restrict__ planes) {
+    build_mip_block(cshift, n_levels, bits, mip, box, planes, blockIdx.x);
 }
 
 // ---- several scenes in one launch ---------------------------------------------------------
@@ -868,7 +992,7 @@ __global__ void __launch_bounds__(256) multi_build_mip_kernel(const __grid_const
     const SceneParams& sp = A.sp[blockIdx.y];
     if (!sp.use_mip || blockIdx.x >= sp.mip_blocks) return;  // whole blocks leave together
     build_mip_block(sp.cshift, sp.a.g.n_levels, reinterpret_cast<const uint4*>(sp.a.g.bits), sp.mip, sp.box,
-                    const_cast<uint32_t*>(sp.cg.planes), sp.cg.plane_words, blockIdx.x);
+                    const_cast<uint32_t*>(sp.cg.planes), blockIdx.x);
 }
 
 __global__ void __launch_bounds__(COUNT_GROUP_MAX)
@@ -880,6 +1004,8 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* spread = reinterpret_cast<uint32_t*>(smem);
     uint8_t* mip = smem + (size_t)12 * A.spread_res;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(
+        mip + (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) + 4 * COUNT_DEPTH_MULTI * threadIdx.x);
     __shared__ float ubox_s[6];
     __shared__ int cut_s;
     __shared__ uint32_t chunk_s;
@@ -933,10 +1059,19 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
                 float* sl = slots ? slots + (size_t)i * slot_cap : nullptr;
                 const uint32_t sc = slots ? slot_cap : 0u;
                 if (meets) {
-                    if (sp.use_mip)
-                        cnt = count_ray<0, true>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, sl, sc);
-                    else
-                        cnt = count_ray<0, false>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, sl, sc);
+                    switch (sp.cg.mode) {  // the same for the whole chunk
+                        case COUNT_POW2:
+                            cnt = count_ray<COUNT_POW2, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            break;
+                        case COUNT_BOUNDED:
+                            cnt = count_ray<COUNT_BOUNDED, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            break;
+                        case COUNT_MIP:
+                            cnt = count_ray<COUNT_MIP, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            break;
+                        default:
+                            cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                    }
                 }
                 if (cnt == 0) alive[i] = 0;
             }
@@ -1156,27 +1291,41 @@ static int make_march_args(const tn_grid_desc* grid, const uint8_t* bitfield, co
 
 // Level-0 constants of the fused count loop, checked against every level of the per-level table
 // (level k must be level 0 scaled by 2^k exactly; base sizes so extreme that this fails are
-// rejected).
+// rejected), and the loop's form (CountMode).
 static int make_count_grid(const MarchArgs& a, CountGrid& cg) {
     const GridView& g = a.g;
-    float half0 = g.half[0];
+    const float half0 = g.half[0], scale0 = g.inv_ls[0] * g.res_f;
     cg.cell0 = g.cell[0];
-    cg.inv_ls0 = g.inv_ls[0];
-    cg.res_f = g.res_f;
+    cg.half_res = 0.5f * g.res_f;
     cg.res_m1 = (uint32_t)(g.res - 1);
     std::memcpy(&cg.half0_bits, &half0, sizeof(int));
     std::memcpy(&cg.cell0_bits, &cg.cell0, sizeof(int));
+    std::memcpy(&cg.scale0_bits, &scale0, sizeof(int));
+    cg.half0_below = cg.half0_bits - (1 << 23);
+    cg.cell0_below = cg.cell0_bits - (1 << 23);
     cg.res_shift = 0;
     while ((1 << cg.res_shift) < g.res) ++cg.res_shift;
-    cg.plane_words = (uint32_t)(((uint64_t)g.res * g.res * g.res) / 32);
-    cg.n_levels = g.n_levels;
+    cg.level_max = g.n_levels - 1;
+    cg.res_below = std::nextafter(g.res_f, 0.0f);
     cg.bits = g.bits;
     cg.planes = nullptr;
+    cg.inv_dt_lo = (float)(1.0 / (double)a.dt_min - (double)a.inv_dt_min);
     for (int k = 0; k < g.n_levels; ++k) {
         const float up = std::ldexp(1.0f, k), dn = std::ldexp(1.0f, -k);
-        TN_REQUIRE(g.half[k] == half0 * up && g.cell[k] == cg.cell0 * up && g.inv_ls[k] == cg.inv_ls0 * dn &&
-                       std::isnormal(half0 * up) && std::isnormal(cg.cell0 * up) && std::isnormal(cg.inv_ls0 * dn),
+        TN_REQUIRE(g.half[k] == half0 * up && g.cell[k] == cg.cell0 * up && g.inv_ls[k] == g.inv_ls[0] * dn &&
+                       std::isnormal(half0 * up) && std::isnormal(cg.cell0 * up) && std::isnormal(g.inv_ls[0] * dn) &&
+                       std::isnormal(scale0 * dn),
                    TN_E_INVALID, "march: base_size %g out of range for %d levels", g.base, g.n_levels);
+    }
+    cg.mode = COUNT_BYTES;
+    if (g.res >= MIP_MIN_RES && g.res <= MIP_MAX_RES) {
+        const tn_bbox& b = a.bbox;
+        float reach = 0.0f;
+        for (float v : {b.min_x, b.min_y, b.min_z, b.max_x, b.max_y, b.max_z}) reach = std::max(reach, std::fabs(v));
+        const float half_last = half0 * std::ldexp(1.0f, g.n_levels - 1);
+        const bool bounded = reach <= half_last;
+        int e;
+        cg.mode = !bounded ? COUNT_MIP : std::frexp(g.inv_ls[0], &e) == 0.5f ? COUNT_POW2 : COUNT_BOUNDED;
     }
     return TN_OK;
 }
@@ -1210,7 +1359,7 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
         chunk += (sc.n_rays + chunk_rays - 1) >> A.chunk_shift;
         const int res = sc.grid.resolution;
         max_res = std::max<uint32_t>(max_res, (uint32_t)res);
-        sp.use_mip = res >= MIP_MIN_RES && res <= MIP_MAX_RES;
+        sp.use_mip = sp.cg.mode != COUNT_BYTES;
         sp.cshift = sp.cg.res_shift - 2;
         if (sp.use_mip) {
             TN_REQUIRE(((uintptr_t)sc.bitfield & 15u) == 0, TN_E_INVALID, "scene %u: bitfield must be 16-byte aligned", s);
@@ -1218,7 +1367,7 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
             sp.mip_blocks = (uint32_t)((mip_bytes + 255) / 256);
             const size_t box_off = (mip_bytes + 255) & ~(size_t)255;
             const size_t planes_off = (box_off + BOX_INTS * sizeof(int) + 255) & ~(size_t)255;
-            const size_t end = planes_off + (size_t)sc.grid.n_levels * sp.cg.plane_words * sizeof(uint32_t);
+            const size_t end = planes_off + sc.grid.n_levels * mip_bytes * sizeof(uint2);
             // pointers are filled once the scratch is allocated
             sp.mip = reinterpret_cast<uint8_t*>(scratch);
             sp.box = reinterpret_cast<int*>(scratch + box_off);
@@ -1254,30 +1403,22 @@ static uint32_t multi_slot_capacity(uint32_t n_rays) {
     return (uint32_t)cap;
 }
 
-template <int NL>
-static int launch_count_nl(bool mip, uint32_t nb, uint32_t group, size_t smem, cudaStream_t stream, const MarchArgs& a,
-                            const CountGrid& cg, uint32_t n_rays, const uint32_t* n_rays_dev, uint32_t rs,
-                            const float* ori, const float* dir, const float* ray_t, const float* ray_t_max,
-                            uint8_t* alive, uint32_t* counts, uint32_t batch_size, uint32_t* batch_info,
-                            uint32_t* block_agg, uint32_t* block_prefix, uint32_t* ticket, uint32_t* flags,
-                            const uint8_t* mip_g, const int* box_g, float* slots, uint32_t slot_cap) {
+template <int MODE>
+static int launch_count(uint32_t nb, uint32_t group, size_t smem, cudaStream_t stream, const MarchArgs& a,
+                        const CountGrid& cg, uint32_t n_rays, const uint32_t* n_rays_dev, uint32_t rs,
+                        const float* ori, const float* dir, const float* ray_t, const float* ray_t_max,
+                        uint8_t* alive, uint32_t* counts, uint32_t batch_size, uint32_t* batch_info,
+                        uint32_t* block_agg, uint32_t* block_prefix, uint32_t* ticket, uint32_t* flags,
+                        const uint8_t* mip_g, const int* box_g, float* slots, uint32_t slot_cap) {
     if (smem > 48 * 1024) {
         // the side_sms reservation: allow the device's opt-in shared memory (set once per kernel)
-        static const int optin_status = [] {
-            const int st = allow_optin_smem((const void*)march_count_kernel<NL, true>);
-            return st == TN_OK ? allow_optin_smem((const void*)march_count_kernel<NL, false>) : st;
-        }();
+        static const int optin_status = allow_optin_smem((const void*)march_count_kernel<MODE>);
         if (optin_status != TN_OK) return optin_status;
     }
-    if (mip)
-        march_count_kernel<NL, true><<<nb, group, smem, stream>>>(
-            a, cg, n_rays, n_rays_dev, rs, ori, dir, ray_t, ray_t_max, alive, counts, batch_size, batch_info,
-            block_agg, block_prefix, ticket, flags, mip_g, box_g, slots, slot_cap);
-    else
-        march_count_kernel<NL, false><<<nb, group, smem, stream>>>(
-            a, cg, n_rays, n_rays_dev, rs, ori, dir, ray_t, ray_t_max, alive, counts, batch_size, batch_info,
-            block_agg, block_prefix, ticket, flags, mip_g, box_g, slots, slot_cap);
-    return TN_OK;
+    march_count_kernel<MODE><<<nb, group, smem, stream>>>(a, cg, n_rays, n_rays_dev, rs, ori, dir, ray_t, ray_t_max,
+                                                          alive, counts, batch_size, batch_info, block_agg,
+                                                          block_prefix, ticket, flags, mip_g, box_g, slots, slot_cap);
+    return check_launch("tn_march_count");
 }
 
 // The two passes of the compaction with a tile of BLOCK x ITEMS values.
@@ -1327,12 +1468,12 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     // coarse mip of the bitfield, the per-level boxes of occupied blocks and the bit-planes:
     // ctx->mip = [mip (R^3/64 B) | box | planes (n_levels x R^3/8 B, 256-byte aligned)]
     const int res = grid->resolution;
-    const bool use_mip = res >= MIP_MIN_RES && res <= MIP_MAX_RES;
+    const bool use_mip = cg.mode != COUNT_BYTES;
     const uint32_t mip_bytes = use_mip ? (uint32_t)(res / 4) * (res / 4) * (res / 4) : 0u;
     const size_t planes_off = ((size_t)mip_bytes + BOX_INTS * sizeof(int) + 255) & ~(size_t)255;
     int* box = nullptr;
     if (use_mip) {
-        st = ensure_mip(ctx, planes_off + (size_t)grid->n_levels * cg.plane_words * sizeof(uint32_t));
+        st = ensure_mip(ctx, planes_off + (size_t)grid->n_levels * mip_bytes * sizeof(uint2));
         if (st != TN_OK) return st;
         TN_REQUIRE(((uintptr_t)bitfield & 15u) == 0, TN_E_INVALID, "bitfield must be 16-byte aligned");
         box = reinterpret_cast<int*>(ctx->mip + mip_bytes);
@@ -1344,7 +1485,7 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
         if (st != TN_OK) return st;
         build_mip_kernel<<<(mip_bytes + 255) / 256, 256, 0, stream>>>(
             cg.res_shift - 2, grid->n_levels, reinterpret_cast<const uint4*>(bitfield), ctx->mip, box,
-            reinterpret_cast<uint32_t*>(ctx->mip + planes_off), cg.plane_words);
+            reinterpret_cast<uint32_t*>(ctx->mip + planes_off));
         st = check_launch("tn_march_count(mip)");
         if (st != TN_OK) return st;
     }
@@ -1354,23 +1495,23 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     if (st != TN_OK) return st;
     ctx->slot_cap = slot_cap;
     ctx->slot_rays = n_rays;
-    size_t smem = (size_t)12 * res + mip_bytes;
+    size_t smem = (use_mip ? mip_bytes : (size_t)12 * res) + (size_t)COUNT_RING * group;
     // with SMs kept for other work, each count block holds its SM alone (see exclusive_smem)
     if (ctx->tune.side_sms) smem = std::max(smem, exclusive_smem());
-#define TN_COUNT_CASE(NL)                                                                                          \
-    case NL:                                                                                                       \
-        st = launch_count_nl<NL>(use_mip, nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t,     \
-                            ray_t_max, alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb, \
-                            ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, box, ctx->slots, slot_cap);       \
-        break;
-    switch (grid->n_levels) {
-        TN_COUNT_CASE(1) TN_COUNT_CASE(2) TN_COUNT_CASE(3) TN_COUNT_CASE(4)
-        TN_COUNT_CASE(5) TN_COUNT_CASE(6) TN_COUNT_CASE(7) TN_COUNT_CASE(8)
+#define TN_COUNT(MODE)                                                                                             \
+    launch_count<MODE>(nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t, ray_t_max, \
+                       alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb,                \
+                       ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, box, ctx->slots, slot_cap)
+    switch (cg.mode) {
+        case COUNT_POW2: st = TN_COUNT(COUNT_POW2); break;
+        case COUNT_BOUNDED: st = TN_COUNT(COUNT_BOUNDED); break;
+        case COUNT_MIP: st = TN_COUNT(COUNT_MIP); break;
+        default: st = TN_COUNT(COUNT_BYTES);
     }
-#undef TN_COUNT_CASE
+#undef TN_COUNT
     if (st != TN_OK) return st;
     ctx->count_group_used = group;
-    return check_launch("tn_march_count");
+    return TN_OK;
 }
 
 int tn_march_emit(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, const uint8_t* bitfield,
@@ -1443,7 +1584,8 @@ int tn_multi_march_count(tn_ctx* ctx, tn_stream_t stream, uint32_t n_scenes, con
         st = check_launch("tn_multi_march_count(mip)");
         if (st != TN_OK) return st;
     }
-    const size_t smem = (size_t)12 * A.spread_res + (size_t)(MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4);
+    const size_t smem = (size_t)12 * A.spread_res + (size_t)(MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) +
+                        (size_t)COUNT_DEPTH_MULTI * 4 * chunk_rays;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, multi_count_kernel, (int)chunk_rays, smem);
     const uint32_t grid = std::min<uint32_t>(A.total_chunks, (uint32_t)(num_sms() * std::max(per_sm, 1)));
