@@ -72,3 +72,52 @@ def test_march_forms(name):
     assert_bitwise(host(off).view(np.uint32), off_o, "offsets")
     for key in ("t", "dt", "m_norm", "dt_norm"):
         assert_bitwise(host(smp[key])[:total].view(np.uint32), em[key][:total].view(np.uint32), key)
+
+
+def _few_alive(n, alive_at, rng):
+    """n rays of which those at alive_at march through the single-cascade scene."""
+    sc = scenes.march_scene_cascaded(n_rays=len(alive_at), n_levels=3)
+    r = scenes.RayBatch(n, n, np.zeros(3 * n, np.float32), np.ones(3 * n, np.float32), np.zeros(n, np.float32),
+                        np.zeros(n, np.float32), np.zeros(n, np.uint8))
+    k = len(alive_at)
+    for c in range(3):
+        r.ori[c * n + alive_at], r.dir[c * n + alive_at] = sc.rays.ori[c * k:(c + 1) * k], sc.rays.dir[c * k:(c + 1) * k]
+    r.t[alive_at], r.t_max[alive_at], r.alive[alive_at] = sc.rays.t, sc.rays.t_max, sc.rays.alive
+    return sc, r
+
+
+@pytest.mark.parametrize("n,rpw", [(4_200_000, 1), (4_200_000, 2), (4_200_000, 4), (300, 1), (300, 4), (5000, 2)])
+def test_emit_past_the_slots_and_in_parts(n, rpw):
+    """4.2 million rays leave 16 step slots a ray, fewer than the marching rays have samples, so the
+    emit pass marches on; a few hundred rays are spread over several warps each."""
+    from turbonerf_b200 import hotpath as hp
+    rng = np.random.default_rng(n)
+    at = np.sort(rng.choice(n, 200, replace=False))
+    sc, r = _few_alive(n, at, rng)
+    march = dict(bbox=sc.bbox, cone=sc.cone_angle, dt_min=sc.dt_min, dt_max=sc.dt_max, max_steps=0)
+    ns_o, alive_o, _ = oracle.march_count(r.as_dict(), sc.grid.as_dict(), march)
+    assert ns_o.max() > 64
+    off_o = np.concatenate([[0], np.cumsum(ns_o[:-1])]).astype(np.uint32)
+    total = int(ns_o.sum())
+    em = oracle.march_emit(r.as_dict(), sc.grid.as_dict(), march, off_o, ns_o, alive_o, n, total, 1.0 / sc.aabb_size)
+    ctx = hp.Context()
+    ctx.tuning = {"emit_rays_per_warp": rpw}
+    g, m = hp.GridSpec(3, 128, 1.0), hp.MarchSpec(sc.cone_angle, sc.dt_min, sc.dt_max, 0)
+    ori, dr, t, tmax, alive = dev(r.ori), dev(r.dir), dev(r.t), dev(r.t_max), dev(r.alive)
+    bits = dev(sc.grid.bitfield)
+    ns, info = hp.march_count(ctx, g, bits, sc.bbox, m, n, n, ori, dr, t, tmax, alive, 0xFFFFFFFF)
+    off, smp = hp.march_emit(ctx, g, bits, sc.bbox, m, 1.0 / sc.aabb_size, n, n, total, info, ori, dr, t, alive, ns)
+    assert ctx.check() == 0
+    assert_bitwise(host(ns).view(np.uint32), ns_o, "n_steps")
+    assert_bitwise(host(off).view(np.uint32), off_o, "offsets")
+    for key in ("t", "pos", "dir", "dt", "m_norm", "dt_norm"):
+        assert_bitwise(host(smp[key]).view(np.uint32), em[key].view(np.uint32), key)
+    # the same rays as one scene of a multi-scene launch
+    table = hp.scene_table([dict(grid=g, bitfield=bits, bbox=sc.bbox, march=m, inv_aabb=1.0 / sc.aabb_size,
+                                 ray_begin=0, n_rays=n)])
+    alive = dev(r.alive)
+    ns2, _, _ = hp.multi_march_count(ctx, table, n, ori, dr, t, tmax, alive)
+    off2, smp2 = hp.multi_march_emit(ctx, table, n, total, ori, dr, t, alive, ns2)
+    assert ctx.check() == 0
+    for key in ("t", "pos", "m_norm"):
+        assert_bitwise(host(smp2[key]).view(np.uint32), em[key].view(np.uint32), "multi " + key)

@@ -155,14 +155,9 @@ int tn_ctx_reserve(tn_ctx* ctx, uint32_t max_rays, uint32_t max_samples) {
     int st = ensure_block_u32(ctx, 2 * blocks);
     if (st == TN_OK) st = ensure_block_f32(ctx, 8 * blocks);
     // march scratch: the 128^3 coarse mip with its occupied boxes and 8 bit-planes (33,024 B +
-    // 8 x 256 KiB), and the step-position slots (16 Mi floats at most)
+    // 8 x 256 KiB), and the step-position slots
     if (st == TN_OK) st = ensure_mip(ctx, 33024u + 8u * 262144u);
-    if (st == TN_OK && max_rays) {
-        size_t per = (16u << 20) / max_rays;
-        if (per > 1024) per = 1024;
-        if (per < 16) per = 16;
-        st = ensure_slots(ctx, per * max_rays);
-    }
+    if (st == TN_OK && max_rays) st = ensure_slots(ctx, (size_t)slot_capacity(max_rays, 0) * max_rays);
     if (st == TN_OK) st = cuda_status(cudaDeviceSynchronize(), "tn_ctx_reserve");
     return st;
 }

@@ -766,47 +766,86 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
+constexpr int EXPAND_U = 4;
+
+// The march of ray r from its occupied step at t on: writes the positions of the next n >= 1 occupied
+// steps (which the count pass found) and returns the last one.
+__device__ float replay_steps(const MarchArgs& a, const RayMarch& r, float t, uint32_t n, float* out) {
+    float last = t;
+    t = __fadd_rn(t, get_dt(t, a.cone, a.dt_min, a.dt_max));
+    // the count pass bounded this loop; the limit only protects against inputs that changed since
+    for (uint32_t taken = 0, iters = 0; taken < n && iters < a.max_iters; ++iters) {
+        float x, y, z;
+        ray_point(r, t, x, y, z);
+        const float dt = get_dt(t, a.cone, a.dt_min, a.dt_max);
+        const int k = grid_level_at(a.g, x, y, z, dt);
+        if (occupied_at(a.g, k, x, y, z)) {
+            out[taken++] = last = t;
+            t = __fadd_rn(t, dt);
+        } else {
+            t = __fadd_rn(t, dt_to_next_voxel(a.g, x, y, z, r.dx, r.dy, r.dz, r.idx, r.idy, r.idz, a.dt_min, k));
+        }
+    }
+    return last;
+}
+
 // Emit pass from the recorded step positions, one warp per ray, so that the rays inside the
 // batch (the first ones) spread over every SM. The warp rebuilds its ray's offset from the
 // group prefix of the count pass plus the counts of the group's earlier rays, writes it, and
 // expands the samples with one lane per sample (coalesced stores of the packed sample arrays).
 // Every value is the one the reference's emit loop (training-batch-kernels.cuh:412-480)
 // computes from the same t: dt = get_dt(t), the position o + t d, m = t + dt/2, the ray's span
-// from its start t to the end of its last step. Rays with more samples than slots fall back to
-// replaying their march.
-// Writes the n samples of ray r_i at o0.. from its recorded step positions (one lane per sample),
-// or, for a ray with more samples than slots, by replaying its march on lane 0.
+// from its start t to the end of its last step.
+// Writes the n samples of ray r_i at o0.. from its recorded step positions, one lane per sample.
+// Where a ray has more samples than slots, its march goes on from the last recorded step on the
+// group's first lane, which leaves the remaining positions in the samples' own t; then all lanes
+// write as before. (The whole march of such a ray on one lane, samples included, took 1.45 ms of a
+// launch over 2.5e5 rays of which 2% have more samples than the 271 slots; this way
+// 0.43 ms. Four positions a lane in flight take 2^16 rays of 195 samples from 217 to 170 us.)
+// `group`: the lanes of this ray, which run this together.
 __device__ __forceinline__ void expand_ray(const MarchArgs& a, float inv_aabb, uint32_t r_i, uint32_t o0, uint32_t n,
                                            uint32_t rs, const uint32_t* __restrict__ img_id,
                                            const float* __restrict__ ori, const float* __restrict__ dir,
                                            const float* __restrict__ ray_t, const SampleOut& o,
                                            const float* __restrict__ slots, uint32_t slot_cap, int lane,
-                                           int lanes) {
+                                           int lanes, unsigned group) {
     RayMarch r;
     load_ray(r, ori, dir, r_i, rs);
     r.t = ray_t[r_i];
     const uint32_t img = img_id ? img_id[r_i] : 0u;
-    if (n > slot_cap) {
-        if (lane == 0) march_emit_ray(a, r, n, o0, img, inv_aabb, o);
-        return;
-    }
     const float* sl = slots + (size_t)r_i * slot_cap;
-    const float t_last = sl[n - 1];
+    const uint32_t kept = min(n, slot_cap);
+    float t_last = sl[kept - 1];
+    if (kept < n) {
+        if (lane == 0) t_last = replay_steps(a, r, t_last, n - kept, o.t + o0 + kept);
+        t_last = __shfl_sync(group, t_last, __ffs(group) - 1);
+        __syncwarp(group);  // the positions written by the first lane
+    }
     const float t_end = __fadd_rn(t_last, get_dt(t_last, a.cone, a.dt_min, a.dt_max));
     const float t_span = fmaxf(__fadd_rn(t_end, -r.t), 1e-6f);
-    for (uint32_t j = lane; j < n; j += lanes) {
-        const float t = sl[j];
+    auto sample = [&](uint32_t s, float t) {
         const float dt = get_dt(t, a.cone, a.dt_min, a.dt_max);
         float x, y, z;
         ray_point(r, t, x, y, z);
-        const uint32_t s = o0 + j;
-        o.t[s] = t;
         const float m = __fadd_rn(t, __fmul_rn(0.5f, dt));
         o.m_norm[s] = clamp_ref(__fdiv_rn(__fadd_rn(m, -r.t), t_span), 0.0f, 1.0f);
         o.dt_norm[s] = __fdiv_rn(dt, t_span);
         if (o.img_id) o.img_id[s] = img;
         write_sample(o, s, x, y, z, r, dt, inv_aabb);
+    };
+    // EXPAND_U positions a lane are loaded before any sample is computed
+    for (uint32_t j = lane; j < kept; j += EXPAND_U * lanes) {
+        float t[EXPAND_U];
+#pragma unroll
+        for (int u = 0; u < EXPAND_U; ++u) t[u] = j + u * lanes < kept ? __ldg(sl + j + u * lanes) : 0.0f;
+#pragma unroll
+        for (int u = 0; u < EXPAND_U; ++u) {
+            if (j + u * lanes >= kept) break;
+            o.t[o0 + j + u * lanes] = t[u];
+            sample(o0 + j + u * lanes, t[u]);
+        }
     }
+    for (uint32_t j = kept + lane; j < n; j += lanes) sample(o0 + j, *((volatile const float*)(o.t + o0 + j)));
 }
 
 constexpr int EXPAND_THREADS_MAX = 512;  // 16 warps (tn_tuning::emit_warps_per_block)
@@ -819,8 +858,8 @@ __device__ __forceinline__ uint32_t group_sum(uint32_t v) {
     return v;
 }
 
-// RPW rays per warp (32 / RPW lanes per ray), blockDim.x / 32 warps per block; the count pass
-// grouped its rays by 2^group_shift (the block size it ran with).
+// RPW rays per warp (32 / RPW lanes per ray), blockDim.x / 32 warps per block, gridDim.y groups of
+// lanes per ray; the count pass grouped its rays by 2^group_shift (the block size it ran with).
 template <int RPW>
 __global__ void __launch_bounds__(EXPAND_THREADS_MAX)
 expand_kernel(MarchArgs a, float inv_aabb, uint32_t n_rays, const uint32_t* __restrict__ n_rays_dev, uint32_t rs,
@@ -843,13 +882,18 @@ expand_kernel(MarchArgs a, float inv_aabb, uint32_t n_rays, const uint32_t* __re
     if (!valid) return;
     const uint32_t o0 = part + block_prefix[r_i >> group_shift];
     const uint32_t n = counts[r_i];
-    if (sub == 0) offsets[r_i] = o0;
+    if (sub == 0 && blockIdx.y == 0) offsets[r_i] = o0;
     if (r_i >= batch_info[0] || n == 0 || !alive[r_i]) return;
     if ((unsigned long long)o0 + n > (unsigned long long)o.ss) {
         if (sub == 0) raise_flag(flags, ERR_CAPACITY);
         return;
     }
-    expand_ray(a, inv_aabb, r_i, o0, n, rs, img_id, ori, dir, ray_t, o, slots, slot_cap, sub, L);
+    // a ray whose march has to go on stays with one group of lanes
+    const bool split = gridDim.y > 1 && n <= slot_cap;
+    if (!split && blockIdx.y > 0) return;
+    expand_ray(a, inv_aabb, r_i, o0, n, rs, img_id, ori, dir, ray_t, o, slots, slot_cap,
+               split ? (int)blockIdx.y * L + sub : sub, split ? (int)gridDim.y * L : L,
+               L == 32 ? FULL_MASK : ((1u << (L & 31)) - 1u) << (lane - sub));
 }
 
 // Bits k of the four bytes of x, Morton cells 4j .. 4j+3 (x0 y0 = 00, 10, 01, 11), at the bits 0, 1,
@@ -1141,7 +1185,8 @@ multi_expand_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const uint
         if (sub == 0) raise_flag(flags, ERR_CAPACITY);
         return;
     }
-    expand_ray(sp.a, sp.inv_aabb, r_i, o0, n, rs, img_id, ori, dir, ray_t, o, slots, slot_cap, sub, L);
+    expand_ray(sp.a, sp.inv_aabb, r_i, o0, n, rs, img_id, ori, dir, ray_t, o, slots, slot_cap, sub, L,
+               L == 32 ? FULL_MASK : ((1u << (L & 31)) - 1u) << (lane - sub));
 }
 
 // ---- compaction: ascending indices of non-zero values ---------------------------------
@@ -1255,10 +1300,11 @@ __global__ void rays_init_kernel(uint32_t n, uint32_t rs, tn_bbox b, float t_far
     alive[i] = 1;
 }
 
-// Budget of the per-ray step-position slots (floats).
-constexpr size_t SLOT_BUDGET = 16u << 20;
+// Per-ray step-position slots within a budget (floats), one scene's and a multi-scene launch's alike:
+// what a ray has beyond them is marched again by one lane of the emit pass, 0.3 us a step.
+constexpr size_t SLOT_BUDGET = 64u << 20;
 
-static uint32_t slot_capacity(uint32_t n_rays, uint32_t max_steps) {
+uint32_t slot_capacity(uint32_t n_rays, uint32_t max_steps) {
     size_t cap = SLOT_BUDGET / (n_rays ? n_rays : 1);
     if (cap > 1024) cap = 1024;
     if (max_steps && cap > max_steps) cap = max_steps;
@@ -1391,16 +1437,6 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
         sp.cg.planes = reinterpret_cast<const uint32_t*>(base + (uintptr_t)sp.cg.planes);
     }
     return TN_OK;
-}
-
-// Per-ray step-position slots of a multi-scene launch (a larger budget than one scene's: the
-// batch holds many more rays).
-constexpr size_t MULTI_SLOT_BUDGET = 64u << 20;
-
-static uint32_t multi_slot_capacity(uint32_t n_rays) {
-    size_t cap = MULTI_SLOT_BUDGET / (n_rays ? n_rays : 1);
-    cap = std::min<size_t>(std::max<size_t>(cap, 16), 1024);
-    return (uint32_t)cap;
 }
 
 template <int MODE>
@@ -1539,7 +1575,11 @@ int tn_march_emit(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, con
     const uint32_t gshift = (uint32_t)__builtin_ctz(group);
     const uint32_t warps = ctx->tune.emit_warps_per_block, rpw = ctx->tune.emit_rays_per_warp;
     const uint32_t per_block = warps * rpw;
-    const uint32_t n_blocks = (n_rays + per_block - 1) / per_block;
+    // A launch of few rays gives each ray several warps, as long as all of them are resident at once
+    // (about 32 an SM): 256 rays of 1024 samples 18 -> 5.5 us with 8 warps a ray.
+    uint32_t split = 1;
+    while (split < 8 && 2 * split * ((n_rays + rpw - 1) / rpw) <= 32u * (uint32_t)num_sms()) split *= 2;
+    const dim3 n_blocks((n_rays + per_block - 1) / per_block, split);
 #define TN_EXPAND(RPW)                                                                                              \
     expand_kernel<RPW><<<n_blocks, warps * WARP, 0, stream>>>(a, inv_aabb_size, n_rays, nullptr, ray_stride, gshift, \
                                                              batch_info, ctx->block_u32 + nb, ray_img_id, ori, dir,  \
@@ -1568,7 +1608,7 @@ int tn_multi_march_count(tn_ctx* ctx, tn_stream_t stream, uint32_t n_scenes, con
     TN_REQUIRE(A.total_rays > 0, TN_E_NO_RAYS, "tn_multi_march_count: no rays");
     st = ensure_block_u32(ctx, 2 * (size_t)A.total_chunks);
     if (st != TN_OK) return st;
-    const uint32_t slot_cap = multi_slot_capacity(A.total_rays);
+    const uint32_t slot_cap = slot_capacity(A.total_rays, 0);
     st = ensure_slots(ctx, (size_t)A.total_rays * slot_cap);
     if (st != TN_OK) return st;
     ctx->slot_cap = slot_cap;
