@@ -81,111 +81,174 @@ __device__ __forceinline__ void hg_cell(float p, float scale, uint32_t res, uint
     f = __fsub_rn(s, fl);
 }
 
-// Corner c (bit 0: x + 1, bit 1: y + 1, bit 2: z + 1) of a cell: its entry and trilinear weight
-// ((w_x w_y) w_z, each 1 - f or f).
-struct HashCorners {
-    uint32_t idx[8];
-    float w[8];
+// A sample's cell at a level and its in-cell coordinates.
+struct HashCell {
+    uint32_t x, y, z;
+    float fx, fy, fz;
 };
 
-__device__ __forceinline__ void hg_corners(const HashLevels& H, int l, float px, float py, float pz, HashCorners& c) {
-    uint32_t ix, iy, iz;
-    float fx, fy, fz;
-    hg_cell(px, H.scale[l], H.res[l], ix, fx);
-    hg_cell(py, H.scale[l], H.res[l], iy, fy);
-    hg_cell(pz, H.scale[l], H.res[l], iz, fz);
-    const float gx = __fsub_rn(1.0f, fx), gy = __fsub_rn(1.0f, fy), gz = __fsub_rn(1.0f, fz);
+__device__ __forceinline__ HashCell hg_locate(const HashLevels& H, int l, float px, float py, float pz) {
+    HashCell c;
+    hg_cell(px, H.scale[l], H.res[l], c.x, c.fx);
+    hg_cell(py, H.scale[l], H.res[l], c.y, c.fy);
+    hg_cell(pz, H.scale[l], H.res[l], c.z, c.fz);
+    return c;
+}
+
+__device__ __forceinline__ bool hg_same(const HashCell& a, const HashCell& b) {
+    return a.x == b.x && a.y == b.y && a.z == b.z;
+}
+
+// Corner k (bit 0: x + 1, bit 1: y + 1, bit 2: z + 1) of a cell: its entry and trilinear weight
+// ((w_x w_y) w_z, each 1 - f or f).
+__device__ __forceinline__ uint32_t hg_corner(const HashLevels& H, int l, const HashCell& c, int k) {
+    return hg_index(H, l, c.x + (k & 1), c.y + ((k >> 1) & 1), c.z + ((k >> 2) & 1));
+}
+
+__device__ __forceinline__ void hg_weights(const HashCell& c, float (&w)[8]) {
+    const float gx = __fsub_rn(1.0f, c.fx), gy = __fsub_rn(1.0f, c.fy), gz = __fsub_rn(1.0f, c.fz);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t bx = k & 1, by = (k >> 1) & 1, bz = (k >> 2) & 1;
-        c.idx[k] = hg_index(H, l, ix + bx, iy + by, iz + bz);
-        c.w[k] = __fmul_rn(__fmul_rn(bx ? fx : gx, by ? fy : gy), bz ? fz : gz);
-    }
+    for (int k = 0; k < 8; ++k)
+        w[k] = __fmul_rn(__fmul_rn((k & 1) ? c.fx : gx, ((k >> 1) & 1) ? c.fy : gy), ((k >> 2) & 1) ? c.fz : gz);
 }
 
 __device__ __forceinline__ uint32_t live_count(uint32_t n, const uint32_t* n_dev) {
     return n_dev ? min(*n_dev, n) : n;
 }
 
+// RUN consecutive values from s0 (those below n; the others zero), as 16-byte groups when VEC.
+template <int RUN, bool VEC>
+__device__ __forceinline__ void hg_load_run(const float* __restrict__ p, uint32_t s0, uint32_t n, float (&v)[RUN]) {
+    if (VEC && s0 + RUN <= n) {
+#pragma unroll
+        for (int q = 0; q < RUN / 4; ++q) {
+            const float4 u = __ldg(reinterpret_cast<const float4*>(p + s0) + q);
+            v[4 * q] = u.x;
+            v[4 * q + 1] = u.y;
+            v[4 * q + 2] = u.z;
+            v[4 * q + 3] = u.w;
+        }
+    } else {
+#pragma unroll
+        for (int q = 0; q < RUN; ++q) v[q] = s0 + q < n ? __ldg(p + s0 + q) : 0.0f;
+    }
+}
+
+constexpr int HG_THREADS = 256;
+
 // One thread per (sample, level): the level's two features, sum over the corners in order of
 // w_c * entry (fused multiply-adds).
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(HG_THREADS)
 hg_encode_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t pstride, uint32_t stride,
                  const float* __restrict__ pos, const float2* __restrict__ params, float* __restrict__ feat) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     const int l = blockIdx.y;
     if (s >= live_count(n, n_dev)) return;
-    HashCorners c;
-    hg_corners(H, l, pos[s], pos[s + pstride], pos[s + 2 * (size_t)pstride], c);
+    const HashCell c = hg_locate(H, l, pos[s], pos[s + pstride], pos[s + 2 * (size_t)pstride]);
     const float2* P = params + ((size_t)l << H.log2_t);
     float2 v[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) v[k] = __ldg(P + c.idx[k]);
+    for (int k = 0; k < 8; ++k) v[k] = __ldg(P + hg_corner(H, l, c, k));
+    float w[8];
+    hg_weights(c, w);
     float a0 = 0.0f, a1 = 0.0f;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        a0 = __fmaf_rn(c.w[k], v[k].x, a0);
-        a1 = __fmaf_rn(c.w[k], v[k].y, a1);
+        a0 = __fmaf_rn(w[k], v[k].x, a0);
+        a1 = __fmaf_rn(w[k], v[k].y, a1);
     }
     feat[(size_t)(HG_F * l) * stride + s] = a0;
     feat[(size_t)(HG_F * l + 1) * stride + s] = a1;
 }
 
-// One thread per (sample, level): w_c * dL/dfeature into the corners' entries; each entry a live
-// sample touches is listed once (the thread whose atomic or set the entry's bit appends l T + idx).
-// Contention is cut three ways: a bit already set is seen with a plain read and skips its atomic;
-// the warp's new entries take one counter atomic for the warp; and on levels of resolution up to
-// HG_SHARE_RES, where neighbouring samples (consecutive along a ray) share corners, the lanes of a
-// warp with the same entry add their contributions in shared memory and one of them makes the
-// atomic add.
-constexpr int HG_BWD_THREADS = 256;
-constexpr uint32_t HG_SHARE_RES = 8192;
-__global__ void __launch_bounds__(HG_BWD_THREADS)
+// grads[e] += v for the four floats of an aligned pair of entries in one reduction.
+__device__ __forceinline__ void red_pair(float2* p, float2 a, float2 b) {
+    asm volatile("red.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(p), "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y)
+                 : "memory");
+}
+
+// Adds a cell's corner sums to the gradients. The two corners of an x edge are neighbours in the
+// table, in one aligned pair, for every second x (directly indexed levels: entry e and e + 1 with e
+// even; hashed levels: x even, where x and x + 1 differ in bit 0 of the hash alone): one 16-byte
+// reduction instead of two 8-byte ones (pairs: the gradients are 16-byte aligned).
+__device__ __forceinline__ void hg_flush(const HashLevels& H, int l, const HashCell& c, const float2 (&g)[8],
+                                         float2* __restrict__ G, bool pairs) {
+#pragma unroll
+    for (int k = 0; k < 8; k += 2) {
+        const uint32_t e0 = hg_corner(H, l, c, k), e1 = hg_corner(H, l, c, k + 1);
+        if (pairs && (e0 ^ e1) == 1u) {
+            const bool up = (e0 & 1u) == 0u;
+            red_pair(G + (e0 & ~1u), up ? g[k] : g[k + 1], up ? g[k + 1] : g[k]);
+        } else {
+            atomicAdd(G + e0, g[k]);
+            atomicAdd(G + e1, g[k + 1]);
+        }
+    }
+}
+
+// One thread per RUN consecutive samples and level: w_c * dL/dfeature summed in registers over the
+// samples of a cell, then added to the corners' entries when the cell changes: samples follow each
+// other along rays, so on the coarse half of the levels most of them stay in their cell. Bound by
+// the L2's reductions (about 150 G a second). 2^18 samples, 16 levels of up to 2048: 85 us (110
+// without the paired reductions), 234 us with one sample a thread and the lanes of a warp that
+// share an entry added up in shared memory; on uniform positions only the pairing remains.
+template <int RUN, bool VEC>
+__global__ void __launch_bounds__(HG_THREADS)
 hg_backward_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t pstride, uint32_t stride,
-                   const float* __restrict__ pos, const float* __restrict__ dfeat, float2* __restrict__ grads,
-                   uint32_t* __restrict__ bits, uint32_t* __restrict__ list, uint32_t* __restrict__ count) {
-    __shared__ float2 share[HG_BWD_THREADS];
+                   const float* __restrict__ pos, const float* __restrict__ dfeat, float2* __restrict__ grads, bool pairs) {
+    const uint32_t s0 = (blockIdx.x * HG_THREADS + threadIdx.x) * RUN;
+    const int l = blockIdx.y;
+    const uint32_t nl = live_count(n, n_dev);
+    if (s0 >= nl) return;
+    float px[RUN], py[RUN], pz[RUN], g0[RUN], g1[RUN];
+    hg_load_run<RUN, VEC>(pos, s0, nl, px);
+    hg_load_run<RUN, VEC>(pos + pstride, s0, nl, py);
+    hg_load_run<RUN, VEC>(pos + 2 * (size_t)pstride, s0, nl, pz);
+    hg_load_run<RUN, VEC>(dfeat + (size_t)(HG_F * l) * stride, s0, nl, g0);
+    hg_load_run<RUN, VEC>(dfeat + (size_t)(HG_F * l + 1) * stride, s0, nl, g1);
+    float2* G = grads + ((size_t)l << H.log2_t);
+    HashCell cur;
+    float2 sum[8];
+#pragma unroll
+    for (int q = 0; q < RUN; ++q) {
+        if (s0 + q >= nl) break;
+        const HashCell c = hg_locate(H, l, px[q], py[q], pz[q]);
+        float w[8];
+        hg_weights(c, w);
+        const bool same = q > 0 && hg_same(c, cur);
+        if (q > 0 && !same) hg_flush(H, l, cur, sum, G, pairs);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const float vx = __fmul_rn(w[k], g0[q]), vy = __fmul_rn(w[k], g1[q]);
+            sum[k].x = same ? sum[k].x + vx : vx;
+            sum[k].y = same ? sum[k].y + vy : vy;
+        }
+        cur = c;
+    }
+    hg_flush(H, l, cur, sum, G, pairs);
+}
+
+// Lists every entry a live sample touches once (the thread whose atomic or sets the entry's bit appends
+// l T + idx), one thread per (sample, level). A bit already set is seen with a plain read and skips
+// its atomic; the lanes of a warp that share an entry send one of them; the warp's new entries
+// take one counter atomic for the warp.
+__global__ void __launch_bounds__(HG_THREADS)
+hg_touch_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t pstride,
+                const float* __restrict__ pos, uint32_t* __restrict__ bits, uint32_t* __restrict__ list,
+                uint32_t* __restrict__ count) {
     const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
     const int l = blockIdx.y;
     const int lane = threadIdx.x & 31;
     const bool live = s < live_count(n, n_dev);
     const unsigned active = __ballot_sync(FULL_MASK, live);  // the warp's lanes that continue together
     if (!live) return;
-    HashCorners c;
-    hg_corners(H, l, pos[s], pos[s + pstride], pos[s + 2 * (size_t)pstride], c);
-    const float g0 = dfeat[(size_t)(HG_F * l) * stride + s], g1 = dfeat[(size_t)(HG_F * l + 1) * stride + s];
+    const HashCell c = hg_locate(H, l, pos[s], pos[s + pstride], pos[s + 2 * (size_t)pstride]);
     const uint32_t base = (uint32_t)l << H.log2_t;
-    const bool share_level = H.res[l] <= HG_SHARE_RES;  // the same for the whole block
-    // the gradient adds of all 8 corners (reductions without a result: nothing waits for them)
-    bool lead[8];
-#pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        float2 v = make_float2(__fmul_rn(c.w[k], g0), __fmul_rn(c.w[k], g1));
-        lead[k] = true;
-        if (share_level) {
-            const unsigned peers = __match_any_sync(active, c.idx[k]);
-            share[threadIdx.x] = v;
-            __syncwarp(active);
-            lead[k] = lane == __ffs(peers) - 1;
-            if (lead[k]) {
-                for (unsigned rest = peers & (peers - 1u); rest; rest &= rest - 1u) {
-                    const float2 o = share[(threadIdx.x & ~31u) + (uint32_t)(__ffs(rest) - 1)];
-                    v.x += o.x;
-                    v.y += o.y;
-                }
-            }
-            __syncwarp(active);
-        }
-        if (lead[k]) atomicAdd(grads + base + c.idx[k], v);
-    }
-    if (!bits) return;
-    // touched entries: every corner's bitmap word read at once, then the atomic ors of the bits
-    // still clear, then one counter atomic for the warp's new entries of all 8 corners
     uint32_t e[8], word[8];
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        e[k] = base + c.idx[k];
-        word[k] = lead[k] ? bits[e[k] >> 5] : ~0u;
+        e[k] = base + hg_corner(H, l, c, k);
+        word[k] = lane == __ffs(__match_any_sync(active, e[k])) - 1 ? bits[e[k] >> 5] : ~0u;
     }
     bool fresh[8];
 #pragma unroll
@@ -293,76 +356,101 @@ hg_heads_forward_kernel(uint32_t nf, uint32_t n, const uint32_t* __restrict__ n_
     }
 }
 
-// One thread per sample: dL/dfeature (written) and the heads' parameter gradients, summed over
-// the block into partials[block][4][HG_MAX_FEAT + 1] (head o's weights j < nf, then its bias at
-// HG_MAX_FEAT; deterministic: fixed lanes, fixed warps).
+// A warp takes 32 samples at a time, a grid apart: a thread per sample for dL/dfeature (written)
+// and dz, then a lane per feature for the heads' parameter gradients, which adds dz_o f_j over the
+// 32 samples from the warp's shared tile; summed over the block into partials[block][4]
+// [HG_MAX_FEAT + 1] (head o's weights j < nf, then its bias at HG_MAX_FEAT; deterministic: fixed
+// samples a warp, fixed lanes, fixed warps). 2^18 samples of the training step, beside a march on
+// 64 SMs: 35 us; with a thread's 33 products through shared memory for every head and column sums
+// by 231 threads 50 us; with all 132 sums in each thread's registers 120 us (spills, 8 warps an
+// SM); 8 features loaded at a time instead of 16 47 us.
 constexpr int HG_HEAD_THREADS = 256;
+constexpr int HG_HEAD_BLOCKS_PER_SM = 4;
+constexpr int HG_HEAD_GROUP = 16;  // features loaded at a time
 constexpr int HG_HEAD_SLOTS = 4 * (HG_MAX_FEAT + 1);
-__global__ void __launch_bounds__(HG_HEAD_THREADS)
+static_assert(HG_MAX_FEAT == WARP, "one feature a lane");
+__global__ void __launch_bounds__(HG_HEAD_THREADS, HG_HEAD_BLOCKS_PER_SM)
 hg_heads_backward_kernel(uint32_t nf, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t stride,
                          const float* __restrict__ feat, const float* __restrict__ head,
                          const float* __restrict__ dL_ddensity, const float* __restrict__ dL_drgb,
                          float* __restrict__ dfeat, float* __restrict__ partials) {
-    __shared__ float rows[HG_HEAD_THREADS * (HG_MAX_FEAT + 1)];
-    __shared__ float runs[HG_HEAD_THREADS];
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+    constexpr int NW = HG_HEAD_THREADS / WARP, PITCH = HG_MAX_FEAT + 1;
+    __shared__ float4 w_s[HG_MAX_FEAT + 1];  // the heads' weights of a feature (zero past nf); last: the biases
+    __shared__ float f_s[NW][WARP * PITCH];
+    __shared__ float4 dz_s[NW][WARP];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const bool live = s < live_count(n, n_dev);
-    float f[HG_MAX_FEAT];
-    float dz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    if (threadIdx.x <= HG_MAX_FEAT) {
+        const uint32_t j = threadIdx.x == HG_MAX_FEAT ? nf : threadIdx.x, h = nf + 1;
+        const bool on = j < nf || threadIdx.x == HG_MAX_FEAT;
+        w_s[threadIdx.x] = on ? make_float4(head[j], head[h + j], head[2 * h + j], head[3 * h + j])
+                              : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    }
+    __syncthreads();
+    const uint32_t nl = live_count(n, n_dev);
+    float* const tile = f_s[wid];
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, bias[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+    const uint32_t step = gridDim.x * HG_HEAD_THREADS;
+    for (uint32_t s0 = blockIdx.x * HG_HEAD_THREADS + wid * WARP; s0 < nl; s0 += step) {  // whole warps
+        const uint32_t s = s0 + lane;
+        const bool live = s < nl;
+        float4 z = w_s[HG_MAX_FEAT];
+#pragma unroll 1
+        for (int j0 = 0; j0 < HG_MAX_FEAT; j0 += HG_HEAD_GROUP) {
+            float f[HG_HEAD_GROUP];
 #pragma unroll
-    for (int j = 0; j < HG_MAX_FEAT; ++j) f[j] = live && j < (int)nf ? feat[(size_t)j * stride + s] : 0.0f;
-    if (live) {
-        float z[3];
+            for (int j = 0; j < HG_HEAD_GROUP; ++j)
+                f[j] = live && j0 + j < (int)nf ? __ldg(feat + (size_t)(j0 + j) * stride + s) : 0.0f;
 #pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            z[c] = __ldg(head + (c + 1) * (nf + 1) + nf);
-#pragma unroll
-            for (int j = 0; j < HG_MAX_FEAT; ++j)
-                if (j < (int)nf) z[c] = fmaf(__ldg(head + (c + 1) * (nf + 1) + j), f[j], z[c]);
-        }
-        dz[0] = dL_ddensity[s];
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-            const float y = sigmoid(z[c]);
-            dz[c + 1] = dL_drgb[(size_t)c * stride + s] * y * (1.0f - y);
-        }
-#pragma unroll
-        for (int j = 0; j < HG_MAX_FEAT; ++j) {
-            if (j < (int)nf) {
-                float g = 0.0f;
-#pragma unroll
-                for (int o = 0; o < 4; ++o) g = fmaf(dz[o], __ldg(head + o * (nf + 1) + j), g);
-                dfeat[(size_t)j * stride + s] = g;
+            for (int j = 0; j < HG_HEAD_GROUP; ++j) {
+                const float4 w = w_s[j0 + j];
+                z.y = fmaf(w.y, f[j], z.y);
+                z.z = fmaf(w.z, f[j], z.z);
+                z.w = fmaf(w.w, f[j], z.w);
+                tile[lane * PITCH + j0 + j] = f[j];
             }
         }
+        float4 dz = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (live) {
+            const float yr = sigmoid(z.y), yg = sigmoid(z.z), yb = sigmoid(z.w);
+            dz = make_float4(dL_ddensity[s], dL_drgb[s] * yr * (1.0f - yr), dL_drgb[(size_t)stride + s] * yg * (1.0f - yg),
+                             dL_drgb[2 * (size_t)stride + s] * yb * (1.0f - yb));
+        }
+        dz_s[wid][lane] = dz;
+#pragma unroll 8
+        for (int j = 0; j < HG_MAX_FEAT; ++j) {
+            const float4 w = w_s[j];
+            const float g = fmaf(dz.w, w.w, fmaf(dz.z, w.z, fmaf(dz.y, w.y, dz.x * w.x)));
+            if (live && j < (int)nf) dfeat[(size_t)j * stride + s] = g;
+        }
+        bias[0] += dz.x;
+        bias[1] += dz.y;
+        bias[2] += dz.z;
+        bias[3] += dz.w;
+        __syncwarp();
+#pragma unroll 8
+        for (int i = 0; i < WARP; ++i) {
+            const float v = tile[i * PITCH + lane];
+            const float4 d = dz_s[wid][i];
+            acc[0] = fmaf(d.x, v, acc[0]);
+            acc[1] = fmaf(d.y, v, acc[1]);
+            acc[2] = fmaf(d.z, v, acc[2]);
+            acc[3] = fmaf(d.w, v, acc[3]);
+        }
+        __syncwarp();
     }
-    // the block's sums of dz_o f_j and dz_o, one head at a time: each thread's 33 values to a shared
-    // row; 7 groups of threads sum each column over a run of rows; 33 threads add the runs (the
-    // order is fixed)
-    constexpr int NC = HG_MAX_FEAT + 1;
-    constexpr int NG = HG_HEAD_THREADS / NC, RPG = (HG_HEAD_THREADS + NG - 1) / NG;
 #pragma unroll
     for (int o = 0; o < 4; ++o) {
-#pragma unroll
-        for (int j = 0; j < NC; ++j) rows[threadIdx.x * NC + j] = j < HG_MAX_FEAT ? dz[o] * f[j] : dz[o];
-        __syncthreads();
-        if (threadIdx.x < NG * NC) {
-            const int c = threadIdx.x % NC, g = threadIdx.x / NC;
-            float v = 0.0f;
-            for (int t = g * RPG; t < min((g + 1) * RPG, HG_HEAD_THREADS); ++t) v += rows[t * NC + c];
-            runs[g * NC + c] = v;
-        }
-        __syncthreads();
-        if (threadIdx.x < NC) {
-            float v = 0.0f;
-            for (int g = 0; g < NG; ++g) v += runs[g * NC + threadIdx.x];
-            partials[(size_t)blockIdx.x * HG_HEAD_SLOTS + o * NC + threadIdx.x] = v;
-        }
-        __syncthreads();
+        const float b = warp_sum(bias[o]);
+        tile[o * PITCH + lane] = acc[o];
+        if (lane == 0) tile[o * PITCH + HG_MAX_FEAT] = b;
     }
-    (void)lane;
-    (void)wid;
+    __syncthreads();
+    for (int i = threadIdx.x; i < HG_HEAD_SLOTS; i += HG_HEAD_THREADS) {
+        float v = 0.0f;
+#pragma unroll
+        for (int w = 0; w < NW; ++w) v += f_s[w][i];
+        partials[(size_t)blockIdx.x * HG_HEAD_SLOTS + i] = v;
+    }
 }
 
 // The heads' gradients (head o, weight j < nf at o (nf + 1) + j, bias at o (nf + 1) + nf): one
@@ -388,14 +476,22 @@ hg_heads_grad_finish_kernel(uint32_t nf, uint32_t n_blocks, const float* __restr
     }
 }
 
+// 16-byte groups: the base 16-byte aligned and the stride between rows a multiple of 4.
+static bool hg_vec(const void* a, uint32_t a_stride, const void* b, uint32_t b_stride) {
+    return ((((uintptr_t)a | (uintptr_t)b) & 15u) == 0) && ((a_stride | b_stride) & 3u) == 0;
+}
+
+static dim3 hg_grid(uint32_t n, uint32_t levels, int run) {
+    return dim3((n + HG_THREADS * run - 1) / (HG_THREADS * run), levels);
+}
+
 int hashgrid_encode(cudaStream_t stream, const tn_hashgrid_desc* desc, uint32_t n, const uint32_t* n_dev,
                     uint32_t pstride, uint32_t stride, const float* pos, const float* params, float* features) {
     HashLevels H;
     int st = hash_levels(desc, H);
     if (st != TN_OK || n == 0) return st;
-    const dim3 grid((n + 255) / 256, H.n_levels);
-    hg_encode_kernel<<<grid, 256, 0, stream>>>(H, n, n_dev, pstride, stride, pos,
-                                               reinterpret_cast<const float2*>(params), features);
+    hg_encode_kernel<<<hg_grid(n, H.n_levels, 1), HG_THREADS, 0, stream>>>(
+        H, n, n_dev, pstride, stride, pos, reinterpret_cast<const float2*>(params), features);
     return check_launch("tn_hashgrid_encode");
 }
 
@@ -405,10 +501,26 @@ int hashgrid_backward(cudaStream_t stream, const tn_hashgrid_desc* desc, uint32_
     HashLevels H;
     int st = hash_levels(desc, H);
     if (st != TN_OK || n == 0) return st;
-    const dim3 grid((n + HG_BWD_THREADS - 1) / HG_BWD_THREADS, H.n_levels);
-    hg_backward_kernel<<<grid, HG_BWD_THREADS, 0, stream>>>(H, n, n_dev, pstride, stride, pos, dL_dfeatures,
-                                                 reinterpret_cast<float2*>(grads), touched_bits, touched_list,
-                                                 touched_count);
+    const bool pairs = ((uintptr_t)grads & 15u) == 0;
+    float2* G = reinterpret_cast<float2*>(grads);
+    const bool vec = hg_vec(pos, pstride, dL_dfeatures, stride);
+#define TN_HG_BACKWARD(RUN, VEC)                                                                           \
+    hg_backward_kernel<RUN, VEC><<<hg_grid(n, H.n_levels, RUN), HG_THREADS, 0, stream>>>(H, n, n_dev, pstride, \
+                                                                                       stride, pos, dL_dfeatures, G, pairs)
+    // Eight samples a thread from 2^20 (sample, level) pairs on (2^18 samples, 16 levels: 85 us against
+    // 89 with four), four below, where the GPU wants more threads (8000 samples: 5.9 against 9.1 us;
+    // even at 64,000).
+    if ((uint64_t)n * H.n_levels >= (1u << 20)) {
+        if (vec) TN_HG_BACKWARD(8, true);
+        else TN_HG_BACKWARD(8, false);
+    } else {
+        if (vec) TN_HG_BACKWARD(4, true);
+        else TN_HG_BACKWARD(4, false);
+    }
+#undef TN_HG_BACKWARD
+    if (touched_bits)
+        hg_touch_kernel<<<hg_grid(n, H.n_levels, 1), HG_THREADS, 0, stream>>>(H, n, n_dev, pstride, pos, touched_bits,
+                                                                            touched_list, touched_count);
     return check_launch("tn_hashgrid_backward");
 }
 
@@ -441,6 +553,11 @@ struct HashNet {
         cudaFree(list); cudaFree(count);
     }
 };
+
+// Blocks of the heads' backward over up to n samples: all resident at once.
+static uint32_t heads_blocks(uint32_t n) {
+    return std::min((n + HG_HEAD_THREADS - 1) / HG_HEAD_THREADS, (uint32_t)(num_sms() * HG_HEAD_BLOCKS_PER_SM));
+}
 
 static const float* head_params(const HashNet* h) { return h->params + h->n_hash; }
 
@@ -480,7 +597,7 @@ static int hashnet_backward(void* user, tn_stream_t stream, uint32_t n, const ui
     int st = cuda_status(cudaMemsetAsync(param_grads, 0, h->n_hash * sizeof(float), s), "hash-grid gradients");
     if (st == TN_OK) st = cuda_status(cudaMemsetAsync(h->count, 0, sizeof(uint32_t), s), "hash-grid count");
     if (st != TN_OK || n == 0) return st;
-    const uint32_t blocks = (n + HG_HEAD_THREADS - 1) / HG_HEAD_THREADS;
+    const uint32_t blocks = heads_blocks(n);
     hg_heads_backward_kernel<<<blocks, HG_HEAD_THREADS, 0, s>>>(h->n_features, n, n_dev, stride, h->feat,
                                                                 head_params(h), dL_ddensity, dL_drgb, h->dfeat,
                                                                 h->partials);
@@ -516,7 +633,7 @@ int hashnet_create(const tn_hashgrid_desc* desc, const float* params, uint32_t c
     h->cap = cap;
     h->qcap = std::max(qcap, 1u);
     const uint64_t entries = h->n_hash / HG_F;
-    const uint32_t blocks = (cap + HG_HEAD_THREADS - 1) / HG_HEAD_THREADS;
+    const uint32_t blocks = heads_blocks(cap);
     st = cuda_status(cudaMalloc(&h->feat, (size_t)h->n_features * cap * sizeof(float)), "hash-grid features");
     if (st == TN_OK) st = cuda_status(cudaMalloc(&h->dfeat, (size_t)h->n_features * cap * sizeof(float)), "hash-grid dfeat");
     if (st == TN_OK)

@@ -461,13 +461,17 @@ __device__ __forceinline__ float box_exit_t(const tn_bbox& b, const RayMarch& r,
 // Bound: issue and dependent latency of one warp a scheduler, about 100 instructions and 190 cycles
 // a step (600 with the lookup on the chain). The kernel alone on B200: 2^14 rays through 5 cascades
 // of 128^3 164 -> 77 us, 256 rays of 1024 samples through one cascade 314 -> 121 us, sixteen scenes
-// of 2.5e5 rays (persistent launch, many warps a scheduler) 1238 -> 730 us. Depths measured on
-// the first two: 3 84 and 158 us, 4 83 and 140, 5 78 and 134, 6 76 and 129, 8 78 and 118; on the
-// scenes 3 is the best. Words kept in registers instead of shared memory cost 10% (the loads then
+// of 2.5e5 rays (persistent launch, many warps a scheduler) 1238 -> 730 us. Steps in flight (D) on
+// the first two: 3 84 and 158 us, 4 83 and 140, 5 78 and 134, 6 76 and 129, 8 78 and 118. Words kept in registers instead of shared memory cost 10% (the loads then
 // share the few scoreboards and wait for each other).
-constexpr int COUNT_DEPTH = 6;        // steps in flight, one launch a batch
+// Steps in flight: 6 where the launch has the GPU to itself; 3 where it shares it with other work
+// (side_sms: blocks of 256 rays on a part of the SMs; the persistent launch), where other warps
+// hide the lookups and what a wrong guess wastes counts: a training step over a grid of random
+// cells (36% occupied) takes its count 449 us with 3 and 532 with 6, over smooth fields 160 and
+// 179. Alone, 6 wins or ties from 64 to 65,536 rays (2^16: 217 against 265 us).
+constexpr int COUNT_DEPTH = 6;
+constexpr int COUNT_DEPTH_SHARED = 3;
 constexpr int COUNT_RING = 4 * (COUNT_DEPTH | 1);  // bytes a thread of shared memory (an odd number of words: no bank conflicts)
-constexpr int COUNT_DEPTH_MULTI = 3;  // of the persistent launch, which has warps to hide the lookups behind
 
 // Copies the word at p into shared memory asynchronously, or zero when `bytes` is 0 instead of 4.
 __device__ __forceinline__ void fetch_word(uint32_t dst, const uint32_t* p, uint32_t bytes) {
@@ -698,7 +702,7 @@ __device__ __forceinline__ bool ray_box_exit(const RayMarch& r, const float* u, 
 // mip (R^3/64 bytes; the fine test reads the per-level bit-planes), or without it the three Morton
 // spread tables (3 R words). The last block to finish scans the group totals and applies the batch
 // cut on the device.
-template <int MODE>
+template <int MODE, int D>
 __global__ void __launch_bounds__(COUNT_GROUP_MAX)
 march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* __restrict__ n_rays_dev, uint32_t rs,
                    const float* __restrict__ ori, const float* __restrict__ dir, const float* __restrict__ ray_t,
@@ -751,7 +755,7 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
             const float below = nextafterf(t_max, -INFINITY);
             const float t_lim = t_stop < below ? t_stop : below;  // a NaN t_max stays NaN
             if (meets)
-                cnt = count_ray<MODE, COUNT_DEPTH>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip, spread, ring,
+                cnt = count_ray<MODE, D>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip, spread, ring,
                                       slots ? slots + (size_t)i * slot_cap : nullptr, slots ? slot_cap : 0u);
             if (cnt == 0) alive[i] = 0;
         }
@@ -1049,7 +1053,7 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
     uint32_t* spread = reinterpret_cast<uint32_t*>(smem);
     uint8_t* mip = smem + (size_t)12 * A.spread_res;
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(
-        mip + (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) + 4 * COUNT_DEPTH_MULTI * threadIdx.x);
+        mip + (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) + 4 * COUNT_DEPTH_SHARED * threadIdx.x);
     __shared__ float ubox_s[6];
     __shared__ int cut_s;
     __shared__ uint32_t chunk_s;
@@ -1105,16 +1109,16 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
                 if (meets) {
                     switch (sp.cg.mode) {  // the same for the whole chunk
                         case COUNT_POW2:
-                            cnt = count_ray<COUNT_POW2, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_POW2, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                             break;
                         case COUNT_BOUNDED:
-                            cnt = count_ray<COUNT_BOUNDED, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_BOUNDED, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                             break;
                         case COUNT_MIP:
-                            cnt = count_ray<COUNT_MIP, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_MIP, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                             break;
                         default:
-                            cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_MULTI>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                     }
                 }
                 if (cnt == 0) alive[i] = 0;
@@ -1439,7 +1443,7 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
     return TN_OK;
 }
 
-template <int MODE>
+template <int MODE, int D>
 static int launch_count(uint32_t nb, uint32_t group, size_t smem, cudaStream_t stream, const MarchArgs& a,
                         const CountGrid& cg, uint32_t n_rays, const uint32_t* n_rays_dev, uint32_t rs,
                         const float* ori, const float* dir, const float* ray_t, const float* ray_t_max,
@@ -1448,12 +1452,13 @@ static int launch_count(uint32_t nb, uint32_t group, size_t smem, cudaStream_t s
                         const uint8_t* mip_g, const int* box_g, float* slots, uint32_t slot_cap) {
     if (smem > 48 * 1024) {
         // the side_sms reservation: allow the device's opt-in shared memory (set once per kernel)
-        static const int optin_status = allow_optin_smem((const void*)march_count_kernel<MODE>);
+        static const int optin_status = allow_optin_smem((const void*)march_count_kernel<MODE, D>);
         if (optin_status != TN_OK) return optin_status;
     }
-    march_count_kernel<MODE><<<nb, group, smem, stream>>>(a, cg, n_rays, n_rays_dev, rs, ori, dir, ray_t, ray_t_max,
-                                                          alive, counts, batch_size, batch_info, block_agg,
-                                                          block_prefix, ticket, flags, mip_g, box_g, slots, slot_cap);
+    march_count_kernel<MODE, D><<<nb, group, smem, stream>>>(a, cg, n_rays, n_rays_dev, rs, ori, dir, ray_t, ray_t_max,
+                                                             alive, counts, batch_size, batch_info, block_agg,
+                                                             block_prefix, ticket, flags, mip_g, box_g, slots,
+                                                             slot_cap);
     return check_launch("tn_march_count");
 }
 
@@ -1534,15 +1539,20 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     size_t smem = (use_mip ? mip_bytes : (size_t)12 * res) + (size_t)COUNT_RING * group;
     // with SMs kept for other work, each count block holds its SM alone (see exclusive_smem)
     if (ctx->tune.side_sms) smem = std::max(smem, exclusive_smem());
-#define TN_COUNT(MODE)                                                                                             \
-    launch_count<MODE>(nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t, ray_t_max, \
-                       alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb,                \
-                       ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, box, ctx->slots, slot_cap)
+#define TN_COUNT(MODE, D)                                                                                            \
+    launch_count<MODE, D>(nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t, ray_t_max, \
+                          alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb,                \
+                          ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, box, ctx->slots, slot_cap)
+    const bool shared = ctx->tune.side_sms != 0;
     switch (cg.mode) {
-        case COUNT_POW2: st = TN_COUNT(COUNT_POW2); break;
-        case COUNT_BOUNDED: st = TN_COUNT(COUNT_BOUNDED); break;
-        case COUNT_MIP: st = TN_COUNT(COUNT_MIP); break;
-        default: st = TN_COUNT(COUNT_BYTES);
+        case COUNT_POW2:
+            st = shared ? TN_COUNT(COUNT_POW2, COUNT_DEPTH_SHARED) : TN_COUNT(COUNT_POW2, COUNT_DEPTH);
+            break;
+        case COUNT_BOUNDED:
+            st = shared ? TN_COUNT(COUNT_BOUNDED, COUNT_DEPTH_SHARED) : TN_COUNT(COUNT_BOUNDED, COUNT_DEPTH);
+            break;
+        case COUNT_MIP: st = TN_COUNT(COUNT_MIP, COUNT_DEPTH_SHARED); break;
+        default: st = TN_COUNT(COUNT_BYTES, COUNT_DEPTH_SHARED);
     }
 #undef TN_COUNT
     if (st != TN_OK) return st;
@@ -1625,7 +1635,7 @@ int tn_multi_march_count(tn_ctx* ctx, tn_stream_t stream, uint32_t n_scenes, con
         if (st != TN_OK) return st;
     }
     const size_t smem = (size_t)12 * A.spread_res + (size_t)(MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) * (MIP_MAX_RES / 4) +
-                        (size_t)COUNT_DEPTH_MULTI * 4 * chunk_rays;
+                        (size_t)COUNT_DEPTH_SHARED * 4 * chunk_rays;
     int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, multi_count_kernel, (int)chunk_rays, smem);
     const uint32_t grid = std::min<uint32_t>(A.total_chunks, (uint32_t)(num_sms() * std::max(per_sm, 1)));
