@@ -119,7 +119,7 @@ typedef struct tn_tuning {
     uint32_t count_rays_per_block;  /* march count, one thread per ray: 32, 64, 128 or 256 (64) */
     uint32_t emit_warps_per_block;  /* march emit: 1, 2, 4, 8 or 16 warps a block (8) */
     uint32_t emit_rays_per_warp;    /* march emit: 1, 2 or 4 rays a warp = 32, 16 or 8 lanes a ray (1) */
-    uint32_t loss_rays_per_block;   /* fused losses, one warp per ray: 2, 4 or 8 (4) */
+    uint32_t loss_rays_per_block;   /* fused losses, one warp per ray: 2, 4 or 8 (4); 2 runs as 4 */
     uint32_t compact_tile;          /* compaction: values a block, 128, 256, 512, 1024 or 2048 (128) */
     uint32_t multi_chunk_rays;      /* multi-scene count: rays per work-stealing chunk, 32..256 (64) */
     uint32_t side_sms;              /* 0 (default) or the SMs kept for work beside the march: every

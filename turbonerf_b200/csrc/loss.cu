@@ -1616,17 +1616,70 @@ __device__ __forceinline__ float exp_neg(float x) { return __expf(-x); }
 // staging buffer, SA_N arrays of RB_PITCH floats. Lane l owns the slots K l .. K l + K - 1,
 // sample j = slot - e; slots outside the ray read as zero (their staged values belong to other
 // rays). `accumulate`: the merged gradient is added to grad_density (else written over it).
-template <bool VEC, int K>
+// COOP: a ray of up to n_warps * 32 K slots over n_warps warps (`group` of the block, which names
+// their barrier), warp `wid` of them with the slots [32 K wid, 32 K (wid + 1)). Each running sum
+// is the warp's own plus the totals of the warps before (after) it, exchanged through `xs`
+// ([COOP_EXCHANGES][COOP_MAX][4]). Such a ray took 37 us on one warp chunk by chunk, four times a
+// short ray, and held up the launch. 2^18 samples: rays of 150-250 samples (some past 253) 37.5 ->
+// 21 us, geometric counts of mean 48 54 -> 36, of mean 128 55 -> 30; 2368 rays of 300 44 -> 25;
+// rays of at most 253 alone stay within 3% of what they took (48 +- 20: 25.8 and 27.3). In a
+// training step over noisy occupancy (rays of up to 738) 74 -> 43. Tried: two rays of up to 128
+// slots a warp (mean 16 60 -> 34, but mean 48 geometric 36 -> 55, where pairs seldom fit).
+constexpr int COOP_MAX = 4;
+constexpr int COOP_EXCHANGES = 10;
+template <bool VEC, int K, bool COOP>
 __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint32_t r, uint32_t o, uint32_t n,
                                                          int lane, float min_t, float inv_nrays, float grad_scale,
                                                          float lambda, const float* __restrict__ target,
                                                          const float* __restrict__ bg, uint32_t rs,
                                                          float* __restrict__ ray_rgba,
                                                          float* __restrict__ grad_density, float* __restrict__ drgb,
-                                                         float& acc_rec, float& acc_dist, float* sm, bool accumulate) {
+                                                         float& acc_rec, float& acc_dist, float* sm, bool accumulate,
+                                                         int wid, int group, int n_warps, float* xs) {
     static_assert(K % 4 == 0 && K <= RB_SPL, "slots are read in 16-byte groups");
-    const uint32_t e = VEC ? (o & 3u) : 0u;
-    const uint32_t j0 = (uint32_t)lane * K - e;  // sample of the lane's first slot (wraps below the ray)
+    const uint32_t e_ray = VEC ? (o & 3u) : 0u;
+    const uint32_t seg = COOP ? (uint32_t)wid * (WARP * K) : 0u;  // the warp's first slot
+    const uint32_t j0 = seg + (uint32_t)lane * K - e_ray;  // sample of the lane's first slot (wraps below the ray)
+    // the warp's samples [os, os + ns) in the batch, the first at slot seg + e
+    const uint32_t e = seg ? 0u : e_ray, os = seg ? o - e_ray + seg : o;
+    const uint32_t ns = COOP ? (e_ray + n > seg ? min(e_ray + n - seg, (uint32_t)(WARP * K)) - e : 0u) : n;
+    // totals of the warps before / after this one, and of all (exchange x; a barrier of the ray's warps)
+    auto exchange = [&](int x, float v0, float v1, float v2, float v3) {
+        if (lane == 0) *reinterpret_cast<float4*>(xs + 4 * (x * COOP_MAX + wid)) = make_float4(v0, v1, v2, v3);
+        asm volatile("bar.sync %0, %1;" ::"r"(1 + group), "r"(n_warps * WARP) : "memory");
+    };
+    auto got = [&](int x, int w) { return *reinterpret_cast<const float4*>(xs + 4 * (x * COOP_MAX + w)); };
+    auto before = [&](int x, float total) {  // total: lane 31's
+        if (!COOP) return 0.0f;
+        exchange(x, __shfl_sync(FULL_MASK, total, WARP - 1), 0.0f, 0.0f, 0.0f);
+        float c = 0.0f;
+        for (int w = 0; w < wid; ++w) c += got(x, w).x;
+        return c;
+    };
+    auto after = [&](int x, float total) {  // total: lane 0's
+        if (!COOP) return 0.0f;
+        exchange(x, __shfl_sync(FULL_MASK, total, 0), 0.0f, 0.0f, 0.0f);
+        float c = 0.0f;
+        for (int w = n_warps - 1; w > wid; --w) c += got(x, w).x;
+        return c;
+    };
+    auto sum4 = [&](int x, float& a, float& b, float& c, float& d) {  // sums over the warps
+        if (!COOP) return;
+        exchange(x, a, b, c, d);
+        a = b = c = d = 0.0f;
+        for (int w = 0; w < n_warps; ++w) {
+            const float4 v = got(x, w);
+            a += v.x;
+            b += v.y;
+            c += v.z;
+            d += v.w;
+        }
+    };
+    auto add_all = [&](float (&v)[K], float c) {
+        if (!COOP) return;
+#pragma unroll
+        for (int q = 0; q < K; ++q) v[q] += c;
+    };
     const size_t ss = S.ss;
     float* const b_sig = sm + SA_SIG * RB_PITCH;
     float* const b_dt = sm + SA_DT * RB_PITCH;
@@ -1639,17 +1692,17 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
     float* const b_gd = sm + SA_GD * RB_PITCH;
     // every input of the ray in flight at once; the per-ray inputs of the loss meanwhile
     __syncwarp();  // the previous ray's write-back reads of the buffers are done
-    stage_slots<VEC>(b_sig, S.density, o, e, n, lane);
-    stage_slots<VEC>(b_dt, S.dt, o, e, n, lane);
-    stage_slots<VEC>(b_r, S.rgb, o, e, n, lane);
-    stage_slots<VEC>(b_g, S.rgb + ss, o, e, n, lane);
-    stage_slots<VEC>(b_b, S.rgb + 2 * ss, o, e, n, lane);
+    stage_slots<VEC>(b_sig, S.density, os, e, ns, lane);
+    stage_slots<VEC>(b_dt, S.dt, os, e, ns, lane);
+    stage_slots<VEC>(b_r, S.rgb, os, e, ns, lane);
+    stage_slots<VEC>(b_g, S.rgb + ss, os, e, ns, lane);
+    stage_slots<VEC>(b_b, S.rgb + 2 * ss, os, e, ns, lane);
     if (lambda > 0.0f) {
-        stage_slots<VEC>(b_dtn, S.dt_norm, o, e, n, lane);
-        stage_slots<VEC>(b_m, S.m_norm, o, e, n, lane);
+        stage_slots<VEC>(b_dtn, S.dt_norm, os, e, ns, lane);
+        stage_slots<VEC>(b_m, S.m_norm, os, e, ns, lane);
     }
-    if (S.t) stage_slots<VEC>(b_t, S.t, o, e, n, lane);
-    if (accumulate) stage_slots<VEC>(b_gd, grad_density, o, e, n, lane);
+    if (S.t) stage_slots<VEC>(b_t, S.t, os, e, ns, lane);
+    if (accumulate) stage_slots<VEC>(b_gd, grad_density, os, e, ns, lane);
     const float gt_r = target[r], gt_g = target[r + rs], gt_b = target[r + 2 * (size_t)rs];
     const float gt_a = target[r + 3 * (size_t)rs];
     const float bg_r = bg[r], bg_g = bg[r + rs], bg_b = bg[r + 2 * (size_t)rs];
@@ -1681,9 +1734,11 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
 #pragma unroll
         for (int q = 0; q < K; ++q) p[q] = sig[q] * dt[q];
         blk_prefix(p, lane);
+        const float cx = before(0, p[K - 1]);
+        add_all(p, cx);
 #pragma unroll
         for (int q = 0; q < K; ++q) T[q] = exp_neg(p[q]);
-        const float t_in = shift_up(T[K - 1], lane, 1.0f);
+        const float t_in = shift_up(T[K - 1], lane, COOP ? exp_neg(cx) : 1.0f);
         int first_q = K;
         float cut_depth = 0.0f;
 #pragma unroll
@@ -1694,10 +1749,20 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
         const unsigned term = __ballot_sync(FULL_MASK, first_q < K);
         if (term) {
             const int fl = __ffs(term) - 1;
-            used = (uint32_t)fl * K + (uint32_t)__shfl_sync(FULL_MASK, first_q, fl) + 1u - e;
+            used = seg + (uint32_t)fl * K + (uint32_t)__shfl_sync(FULL_MASK, first_q, fl) + 1u - e_ray;
             depth = __shfl_sync(FULL_MASK, cut_depth, fl);
         } else {
             depth = __shfl_sync(FULL_MASK, p[K - 1], WARP - 1);
+        }
+        if (COOP) {  // the first warp with a cut decides, else the last warp's depth stands
+            exchange(1, __uint_as_float(used), depth, 0.0f, 0.0f);
+            for (int w = n_warps - 1; w >= 0; --w) {
+                const float4 v = got(1, w);
+                if (w == n_warps - 1 || __float_as_uint(v.x) < n) {
+                    used = __float_as_uint(v.x);
+                    depth = v.y;
+                }
+            }
         }
     }
     float ar = 0.0f, ag = 0.0f, ab = 0.0f, aa = 0.0f;
@@ -1711,10 +1776,11 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
     }
     CompFwd c;
     c.r = warp_sum(ar); c.g = warp_sum(ag); c.b = warp_sum(ab); c.a = warp_sum(aa);
+    sum4(2, c.r, c.g, c.b, c.a);
     c.depth = depth;
     c.used = used;
     const ReconGrad g = recon_grad(c, gt_r, gt_g, gt_b, gt_a, bg_r, bg_g, bg_b, inv_nrays);
-    if (lane == 0) {
+    if (lane == 0 && (!COOP || wid == 0)) {
         if (ray_rgba) {
             ray_rgba[r] = c.r; ray_rgba[r + rs] = c.g; ray_rgba[r + 2 * (size_t)rs] = c.b;
             ray_rgba[r + 3 * (size_t)rs] = c.a;
@@ -1732,7 +1798,12 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
             cu[q] = g.gr * cr[q] + g.gg * cg[q] + g.gb * cb[q] + g.ga;
             su[q] = w[q] * cu[q];
         }
-        const float su_after = blk_suffix(su, lane);
+        float su_after = blk_suffix(su, lane);
+        {
+            const float cs = after(3, su[0]);
+            add_all(su, cs);
+            if (COOP) su_after += cs;
+        }
         float dr[K], dg[K], db[K];
 #pragma unroll
         for (int q = 0; q < K; ++q) {
@@ -1763,9 +1834,11 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
 #pragma unroll
             for (int q = 0; q < K; ++q) p[q] = sig[q] * dtn[q];
             blk_prefix(p, lane);
+            const float cx = before(4, p[K - 1]);
+            add_all(p, cx);
 #pragma unroll
             for (int q = 0; q < K; ++q) tnext[q] = exp_neg(p[q]);  // T_{j+1}
-            const float t_in = shift_up(tnext[K - 1], lane, 1.0f);
+            const float t_in = shift_up(tnext[K - 1], lane, COOP ? exp_neg(cx) : 1.0f);
 #pragma unroll
             for (int q = 0; q < K; ++q)
                 wd[q] = valid[q] ? (q ? tnext[q - 1] : t_in) * opacity(sig[q] * dtn[q]) : 0.0f;
@@ -1774,9 +1847,15 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
             float W[K];
 #pragma unroll
             for (int q = 0; q < K; ++q) W[q] = wd[q];
-            const float w_before = blk_prefix(W, lane);
+            float w_before = blk_prefix(W, lane);
+            {
+                const float cw = before(5, W[K - 1]);
+                add_all(W, cw);
+                if (COOP) w_before += cw;
+            }
             // m of the previous sample; the first sample has no increment
-            const float m_in = __shfl_up_sync(FULL_MASK, mm[K - 1], 1);
+            float m_in = __shfl_up_sync(FULL_MASK, mm[K - 1], 1);
+            if (COOP && lane == 0 && j0 - 1u < n) m_in = S.m_norm[(size_t)o + j0 - 1u];
 #pragma unroll
             for (int q = 0; q < K; ++q) {
                 const float m_prev = q ? mm[q - 1] : m_in;
@@ -1784,6 +1863,7 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
                 A[q] = dm[q] * (q ? W[q - 1] : w_before);
             }
             blk_prefix(A, lane);
+            add_all(A, before(6, A[K - 1]));
         }
         float uni = 0.0f, cross = 0.0f;
 #pragma unroll
@@ -1796,10 +1876,16 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
 #pragma unroll
         for (int q = 0; q < K; ++q) Wge[q] = wd[q];
         blk_suffix(Wge, lane);
+        add_all(Wge, after(7, Wge[0]));
         float f[K];
 #pragma unroll
         for (int q = 0; q < K; ++q) f[q] = dm[q] * Wge[q];
-        const float f_after = blk_suffix(f, lane);
+        float f_after = blk_suffix(f, lane);
+        {
+            const float cf = after(8, f[0]);
+            add_all(f, cf);
+            if (COOP) f_after += cf;
+        }
         float gw[K], gq[K];
 #pragma unroll
         for (int q = 0; q < K; ++q) {
@@ -1807,7 +1893,12 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
             gq[q] = k * ((2.0f / 3.0f) * dtn[q] * wd[q] + 2.0f * (A[q] + b));
             gw[q] = gq[q] * wd[q];
         }
-        const float gw_after = blk_suffix(gw, lane);
+        float gw_after = blk_suffix(gw, lane);
+        {
+            const float cg = after(9, gw[0]);
+            add_all(gw, cg);
+            if (COOP) gw_after += cg;
+        }
 #pragma unroll
         for (int q = 0; q < K; ++q) {
             const float gw_ex = q < K - 1 ? gw[q + 1] : gw_after;
@@ -1834,13 +1925,13 @@ __device__ __forceinline__ void train_losses_ray_blocked(const Samples& S, uint3
         write_slots(b_gd, lane, gd);
     }
     __syncwarp();
-    store_slots<VEC>(grad_density, b_gd, o, e, n, lane);
-    store_slots<VEC>(drgb, b_r, o, e, n, lane);
-    store_slots<VEC>(drgb + ss, b_g, o, e, n, lane);
-    store_slots<VEC>(drgb + 2 * ss, b_b, o, e, n, lane);
+    store_slots<VEC>(grad_density, b_gd, os, e, ns, lane);
+    store_slots<VEC>(drgb, b_r, os, e, ns, lane);
+    store_slots<VEC>(drgb + ss, b_g, os, e, ns, lane);
+    store_slots<VEC>(drgb + 2 * ss, b_b, os, e, ns, lane);
 }
 
-// Rays longer than RB_MAX: the same computation over super-chunks of RB_MAX samples in the
+// Rays past COOP_MAX warps: the same computation over super-chunks of RB_MAX samples in the
 // blocked layout. The compositor forward carries its running sums from chunk to chunk; its VJP
 // walks the chunks from the last and rebuilds the transmittance from the ray's optical depth
 // and the suffix sums of sigma * dt, as the chunked path does. The distortion forward keeps each
@@ -1916,7 +2007,7 @@ __device__ __forceinline__ void sc_load_dist(const Samples& S, uint32_t o, uint3
     }
 }
 
-// A ray of more than RB_MAX samples: the same three passes as the blocked path (compositor
+// A ray of more than COOP_MAX RB_MAX slots: the same three passes as the blocked path (compositor
 // forward to the cut, distortion forward, reversed backward with the merge), each over chunks
 // of RB_MAX samples that are staged through the warp's buffer `sm` with cp.async, with the
 // chunk's outputs written back through the buffer in coalesced rows.
@@ -2185,10 +2276,10 @@ __device__ __noinline__ void train_losses_ray_long(const Samples& S, uint32_t r,
     }
 }
 
-// Reconstruction + distortion forward/backward + gradient merge, one warp per ray with its own
-// staging buffer (dynamic shared memory, 10.1 KB a warp); W warps a block (tn_tuning
-// loss_rays_per_block: 2, 4 or 8) and 16 / W blocks an SM (128 registers a thread) keep 16 rays
-// in flight per SM. VEC: 16-byte staging (every sample array 16-byte aligned, stride a multiple
+// Reconstruction + distortion forward/backward + gradient merge, one warp per ray (two or four for
+// rays past 256 or 512 slots) with its own staging buffer (dynamic shared memory, 10.1 KB a warp);
+// W warps a block (tn_tuning loss_rays_per_block: 4 or 8; 2 runs as 4, the warps of the longest
+// shared rays) and 16 / W blocks an SM (128 registers a thread) keep 16 rays in flight per SM. VEC: 16-byte staging (every sample array 16-byte aligned, stride a multiple
 // of 4). The grid is every resident warp (or fewer), each taking rays in turn: a batch of many
 // waves (the rays of several scenes) is one persistent launch.
 template <int W, bool VEC>
@@ -2198,7 +2289,7 @@ train_losses_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint32_t 
                     const uint32_t* __restrict__ inv_from, float grad_scale, float lambda,
                     const float* __restrict__ target, const float* __restrict__ bg, float* __restrict__ ray_rgba,
                     float* __restrict__ grad_density, float* __restrict__ drgb, float* loss_sums, float* partials,
-                    uint32_t* ticket, bool accumulate) {
+                    uint32_t* ticket, bool accumulate, int spread_host) {
     extern __shared__ __align__(16) float stage[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_live = live_rays(n_rays, n_dev);
@@ -2207,17 +2298,56 @@ train_losses_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint32_t 
     const float lam = lambda > 0.0f ? lambda : 0.0f;
     float acc[2] = {0.0f, 0.0f};
     float* const sm = stage + (size_t)wid * SA_N * RB_PITCH;
-    auto one_ray = [&](uint32_t r) {
-        const uint32_t o = offsets[r], n = counts[r];
-        const uint32_t span = n + (VEC ? (o & 3u) : 0u);  // slots the ray takes
+    // The block's rays, numbered k: W consecutive ones a round, or (spread) every gridDim.x-th ray.
+    // Long rays are spread over all blocks; short ones, which share their sectors with their
+    // neighbours, go to a block together. The line is a mean of 128 samples a ray, from the host
+    // (spread_host 0, 1) or, where the live rays are only known here, from the offsets.
+    bool spread = spread_host == 1;
+    if (spread_host > 1 && n_live) spread = (offsets[n_live - 1] + counts[n_live - 1]) / 128u >= n_live;
+    auto block_ray = [&](uint32_t k) {
+        return spread ? blockIdx.x + k * gridDim.x : (blockIdx.x + k / W * gridDim.x) * W + k % W;
+    };
+    auto slots_of = [&](uint32_t o, uint32_t n) { return n + (VEC ? (o & 3u) : 0u); };  // slots the ray takes
+    uint32_t most = 0;  // slots of the longest ray left to several warps
+    for (uint32_t k = wid;; k += W) {
+        const uint32_t r = block_ray(k);
+        if (r >= n_live) break;
+        const uint32_t o = offsets[r], n = counts[r], span = slots_of(o, n);
         if (span <= RB_MAX)
-            train_losses_ray_blocked<VEC, RB_SPL>(S, r, o, n, lane, min_t, inv_nrays, grad_scale, lam, target, bg, rs,
-                                                  ray_rgba, grad_density, drgb, acc[0], acc[1], sm, accumulate);
-        else
+            train_losses_ray_blocked<VEC, RB_SPL, false>(S, r, o, n, lane, min_t, inv_nrays, grad_scale, lam, target, bg,
+                                                         rs, ray_rgba, grad_density, drgb, acc[0], acc[1], sm,
+                                                         accumulate, 0, 0, 1, nullptr);
+        else if (span > COOP_MAX * RB_MAX)
             train_losses_ray_long(S, r, o, n, lane, min_t, inv_nrays, grad_scale, lam, target, bg, rs, ray_rgba,
                                   grad_density, drgb, acc[0], acc[1], sm, accumulate);
-    };
-    for (uint32_t r = blockIdx.x * W + wid; r < n_live; r += gridDim.x * W) one_ray(r);
+        else
+            most = max(most, span);
+    }
+    // The rays of up to 2, then of up to 4 warps, by groups of as many warps of the block.
+    for (int nw = 2; nw <= COOP_MAX; nw *= 2) {
+        if (!__syncthreads_or(most > (uint32_t)nw / 2u * RB_MAX)) break;
+        __shared__ __align__(16) float xs[W / 2][COOP_EXCHANGES * COOP_MAX * 4];
+        const int group = wid / nw, groups = W / nw;
+        uint32_t seen = 0;
+        for (uint32_t k0 = 0; block_ray(k0) < n_live; k0 += WARP) {  // every warp finds the same rays
+            const uint32_t r = block_ray(k0 + lane);
+            uint32_t o = 0, n = 0;
+            if (r < n_live) {
+                o = offsets[r];
+                n = counts[r];
+            }
+            const uint32_t span = slots_of(o, n);
+            unsigned mine = __ballot_sync(FULL_MASK, span > (uint32_t)nw / 2u * RB_MAX && span <= (uint32_t)nw * RB_MAX);
+            for (; mine; mine &= mine - 1u, ++seen) {
+                if ((int)(seen % (uint32_t)groups) != group) continue;
+                const int src = __ffs(mine) - 1;
+                train_losses_ray_blocked<VEC, RB_SPL, true>(
+                    S, __shfl_sync(FULL_MASK, r, src), __shfl_sync(FULL_MASK, o, src), __shfl_sync(FULL_MASK, n, src),
+                    lane, min_t, inv_nrays, grad_scale, lam, target, bg, rs, ray_rgba, grad_density, drgb, acc[0],
+                    acc[1], sm, accumulate, wid % nw, group, nw, xs[group]);
+            }
+        }
+    }
     if (loss_sums) {
         acc[0] *= inv_nrays;
         block_sum_and_finish<2>(acc, partials, ticket, loss_sums, FinishScale{{1.0f, 1.0f}, n_dev, n_rays, 2u});
@@ -2395,9 +2525,10 @@ static int blocks_per_sm(const void* kernel, int threads, size_t dyn_smem = 0) {
     return per_sm;
 }
 
-static int loss_grid(const void* kernel, uint32_t n_rays, int threads = LOSS_THREADS, size_t dyn_smem = 0) {
+static int loss_grid(const void* kernel, uint32_t n_rays, int per_block = LOSS_THREADS, int threads = LOSS_THREADS,
+                     size_t dyn_smem = 0) {
     const int per_sm = blocks_per_sm(kernel, threads, dyn_smem);
-    const uint32_t want = (n_rays + threads / WARP - 1) / (threads / WARP);
+    const uint32_t want = (n_rays + per_block / WARP - 1) / (per_block / WARP);
     const uint32_t cap = (uint32_t)(num_sms() * per_sm);
     return (int)max(1u, min(want, cap));
 }
@@ -2412,13 +2543,15 @@ static int launch_train_losses_v(tn_ctx* ctx, cudaStream_t stream, const tn_ray_
     std::call_once(once, [&] {
         cudaFuncSetAttribute(train_losses_kernel<W, VEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     });
-    const int grid = loss_grid((const void*)train_losses_kernel<W, VEC>, batch->n_rays, W * WARP, smem);
+    const int spread = batch->n_rays_dev ? 2 : (uint64_t)batch->n_rays * 128u <= batch->sample_stride;
+    const int grid = loss_grid((const void*)train_losses_kernel<W, VEC>, batch->n_rays, spread ? WARP : W * WARP,
+                               W * WARP, smem);
     int st = ensure_block_f32(ctx, (size_t)grid * 2);
     if (st != TN_OK) return st;
     train_losses_kernel<W, VEC><<<grid, W * WARP, smem, stream>>>(
         S, batch->n_rays, batch->n_rays_dev, batch->ray_stride, batch->counts, batch->offsets, min_t, inv_nrays,
         inv_from, grad_scale, lambda, target, bg, ray_rgba, grad_density, drgb, loss_sums, ctx->block_f32,
-        ctx->tickets + TICKET_TRAIN, accumulate);
+        ctx->tickets + TICKET_TRAIN, accumulate, spread);
     return check_launch("tn_train_losses");
 }
 
@@ -2556,9 +2689,6 @@ int train_losses(tn_ctx* ctx, cudaStream_t stream, const tn_ray_batch* batch, in
     if (batch->n_rays == 0) return TN_OK;
     Samples S{density, rgb, dt, m_norm, dt_norm, t, batch->sample_stride, activation};
     switch (ctx->tune.loss_rays_per_block) {
-        case 2: return launch_train_losses<2>(ctx, stream, batch, S, min_transmittance, inv_nrays, inv_nrays_from_dev,
-                                              grad_scale, lambda, target_rgba, bg_rgb, ray_rgba, grad_density,
-                                              dL_drgb, loss_sums, accumulate);
         case 8: return launch_train_losses<8>(ctx, stream, batch, S, min_transmittance, inv_nrays, inv_nrays_from_dev,
                                               grad_scale, lambda, target_rgba, bg_rgb, ray_rgba, grad_density,
                                               dL_drgb, loss_sums, accumulate);
