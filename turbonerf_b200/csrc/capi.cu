@@ -124,6 +124,9 @@ int tn_ctx_create(tn_ctx** out) {
     if (st == TN_OK) st = cuda_status(cudaMalloc(&ctx->tickets, TICKET_COUNT * sizeof(uint32_t)), "tn_ctx_create tickets");
     if (st == TN_OK) st = cuda_status(cudaMemset(ctx->flags, 0, sizeof(uint32_t)), "tn_ctx_create memset");
     if (st == TN_OK) st = cuda_status(cudaMemset(ctx->tickets, 0, TICKET_COUNT * sizeof(uint32_t)), "tn_ctx_create memset");
+    if (st == TN_OK) st = cuda_status(cudaMalloc(&ctx->box, BOX_INTS * sizeof(int)), "tn_ctx_create box");
+    if (st == TN_OK) st = cuda_status(cudaMemset(ctx->box, BOX_EMPTY_LO & 0xFF, BOX_INTS / 2 * sizeof(int)), "tn_ctx_create memset");
+    if (st == TN_OK) st = cuda_status(cudaMemset(ctx->box + BOX_INTS / 2, 0, BOX_INTS / 2 * sizeof(int)), "tn_ctx_create memset");
     if (st == TN_OK) st = ensure_block_u32(ctx, 4096);
     if (st == TN_OK) st = ensure_block_f32(ctx, 4096);
     if (st == TN_OK) st = cuda_status(cudaDeviceSynchronize(), "tn_ctx_create sync");
@@ -142,6 +145,7 @@ int tn_ctx_destroy(tn_ctx* ctx) {
     cudaFree(ctx->block_u32);
     cudaFree(ctx->block_f32);
     cudaFree(ctx->mip);
+    cudaFree(ctx->box);
     cudaFree(ctx->slots);
     cudaFree(ctx->render_ws);
     delete ctx;
@@ -154,7 +158,7 @@ int tn_ctx_reserve(tn_ctx* ctx, uint32_t max_rays, uint32_t max_samples) {
     const size_t blocks = (size_t)max_rays / 32 + (size_t)max_samples / 1024 + 1024;
     int st = ensure_block_u32(ctx, 2 * blocks);
     if (st == TN_OK) st = ensure_block_f32(ctx, 8 * blocks);
-    // march scratch: the 128^3 coarse mip with its occupied boxes and 8 bit-planes (33,024 B +
+    // march scratch: the 128^3 coarse mip and 8 bit-planes (33,024 B +
     // 8 x 256 KiB), and the step-position slots
     if (st == TN_OK) st = ensure_mip(ctx, 33024u + 8u * 262144u);
     if (st == TN_OK && max_rays) st = ensure_slots(ctx, (size_t)slot_capacity(max_rays, 0) * max_rays);

@@ -323,7 +323,6 @@ constexpr int COUNT_GROUP_MAX = 256;  // largest count block (tn_tuning::count_r
 // The coarse mip (one byte per 4x4x4 block) is staged in shared memory for 16 <= R <= 128.
 constexpr int MIP_MIN_RES = 16;
 constexpr int MIP_MAX_RES = 128;
-constexpr int BOX_INTS = 2 * MAX_LEVELS * 3;  // per level: lo block x,y,z | hi block + 1 x,y,z
 
 __device__ __forceinline__ float pow2i(int e) { return __int_as_float((127 + e) << 23); }
 
@@ -709,7 +708,7 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
                    const float* __restrict__ ray_t_max, uint8_t* __restrict__ alive, uint32_t* counts,
                    uint32_t batch_size, uint32_t* batch_info, uint32_t* block_agg, uint32_t* block_prefix,
                    uint32_t* ticket, uint32_t* flags, const uint8_t* __restrict__ mip_g,
-                   const int* __restrict__ box_g, float* __restrict__ slots, uint32_t slot_cap) {
+                   int* box_g, float* __restrict__ slots, uint32_t slot_cap) {
     constexpr bool MIP = MODE != COUNT_BYTES;
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* spread = reinterpret_cast<uint32_t*>(smem);
@@ -1449,7 +1448,7 @@ static int launch_count(uint32_t nb, uint32_t group, size_t smem, cudaStream_t s
                         const float* ori, const float* dir, const float* ray_t, const float* ray_t_max,
                         uint8_t* alive, uint32_t* counts, uint32_t batch_size, uint32_t* batch_info,
                         uint32_t* block_agg, uint32_t* block_prefix, uint32_t* ticket, uint32_t* flags,
-                        const uint8_t* mip_g, const int* box_g, float* slots, uint32_t slot_cap) {
+                        const uint8_t* mip_g, int* box_g, float* slots, uint32_t slot_cap) {
     if (smem > 48 * 1024) {
         // the side_sms reservation: allow the device's opt-in shared memory (set once per kernel)
         static const int optin_status = allow_optin_smem((const void*)march_count_kernel<MODE, D>);
@@ -1506,26 +1505,19 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     const uint32_t nb = (n_rays + group - 1) / group;
     st = ensure_block_u32(ctx, 2 * (size_t)nb);
     if (st != TN_OK) return st;
-    // coarse mip of the bitfield, the per-level boxes of occupied blocks and the bit-planes:
-    // ctx->mip = [mip (R^3/64 B) | box | planes (n_levels x R^3/8 B, 256-byte aligned)]
+    // coarse mip of the bitfield, the per-level boxes of occupied blocks (ctx->box) and the bit-planes:
+    // ctx->mip = [mip (R^3/64 B) | planes (n_levels x R^3/8 B, 256-byte aligned)]
     const int res = grid->resolution;
     const bool use_mip = cg.mode != COUNT_BYTES;
     const uint32_t mip_bytes = use_mip ? (uint32_t)(res / 4) * (res / 4) * (res / 4) : 0u;
-    const size_t planes_off = ((size_t)mip_bytes + BOX_INTS * sizeof(int) + 255) & ~(size_t)255;
-    int* box = nullptr;
+    const size_t planes_off = ((size_t)mip_bytes + 255) & ~(size_t)255;
     if (use_mip) {
         st = ensure_mip(ctx, planes_off + (size_t)grid->n_levels * mip_bytes * sizeof(uint2));
         if (st != TN_OK) return st;
         TN_REQUIRE(((uintptr_t)bitfield & 15u) == 0, TN_E_INVALID, "bitfield must be 16-byte aligned");
-        box = reinterpret_cast<int*>(ctx->mip + mip_bytes);
         cg.planes = reinterpret_cast<const uint32_t*>(ctx->mip + planes_off);
-        st = cuda_status(cudaMemsetAsync(box, 0x7f, BOX_INTS / 2 * sizeof(int), stream), "tn_march_count(box)");
-        if (st == TN_OK)
-            st = cuda_status(cudaMemsetAsync(box + BOX_INTS / 2, 0, BOX_INTS / 2 * sizeof(int), stream),
-                             "tn_march_count(box)");
-        if (st != TN_OK) return st;
         build_mip_kernel<<<(mip_bytes + 255) / 256, 256, 0, stream>>>(
-            cg.res_shift - 2, grid->n_levels, reinterpret_cast<const uint4*>(bitfield), ctx->mip, box,
+            cg.res_shift - 2, grid->n_levels, reinterpret_cast<const uint4*>(bitfield), ctx->mip, ctx->box,
             reinterpret_cast<uint32_t*>(ctx->mip + planes_off));
         st = check_launch("tn_march_count(mip)");
         if (st != TN_OK) return st;
@@ -1542,7 +1534,7 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
 #define TN_COUNT(MODE, D)                                                                                            \
     launch_count<MODE, D>(nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t, ray_t_max, \
                           alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb,                \
-                          ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, box, ctx->slots, slot_cap)
+                          ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, ctx->box, ctx->slots, slot_cap)
     const bool shared = ctx->tune.side_sms != 0;
     switch (cg.mode) {
         case COUNT_POW2:

@@ -367,22 +367,28 @@ int launch_occupancy_update(tn_ctx* ctx, cudaStream_t stream, const tn_grid_desc
     return check_launch("tn_occupancy_update(densities)");
 }
 
-int launch_occupancy_bits_ahead(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
-                                const uint8_t* bitfield, uint8_t* bitfield_out, uint32_t n_updates,
-                                const int32_t* levels, const uint32_t* cells, const float* values,
-                                const float* rand_select, int activation, const uint32_t* sample_all_dev, float decay,
-                                float threshold) {
+int launch_occupancy_bits_decayed(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
+                                  uint8_t* bitfield_out, float decay, float threshold) {
     int st = validate_grid(grid);
     if (st != TN_OK) return st;
-    TN_NONNULL(density); TN_NONNULL(bitfield); TN_NONNULL(bitfield_out); TN_NONNULL(sample_all_dev);
+    TN_NONNULL(density); TN_NONNULL(bitfield_out);
     TN_REQUIRE(((uintptr_t)density & 15u) == 0 && ((uintptr_t)bitfield_out & 3u) == 0, TN_E_INVALID,
                "occupancy bits ahead: density must be 16-byte and bitfield 4-byte aligned");
-    const uint32_t volume = (uint32_t)grid->resolution * grid->resolution * grid->resolution;
-    const uint32_t v4 = volume / 4;
+    const uint32_t v4 = (uint32_t)grid->resolution * grid->resolution * grid->resolution / 4;
     occ_bits_decayed_kernel<<<(v4 + 255) / 256, 256, 0, stream>>>(v4, grid->n_levels, density, bitfield_out, decay,
                                                                    threshold);
-    st = check_launch("occupancy bits ahead (decayed)");
+    return check_launch("occupancy bits ahead (decayed)");
+}
+
+int launch_occupancy_bits_raised(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
+                                 const uint8_t* bitfield, uint8_t* bitfield_out, uint32_t n_updates,
+                                 const int32_t* levels, const uint32_t* cells, const float* values,
+                                 const float* rand_select, int activation, const uint32_t* sample_all_dev, float decay,
+                                 float threshold) {
+    int st = validate_grid(grid);
     if (st != TN_OK || n_updates == 0) return st;
+    TN_NONNULL(density); TN_NONNULL(bitfield); TN_NONNULL(bitfield_out); TN_NONNULL(sample_all_dev);
+    const uint32_t volume = (uint32_t)grid->resolution * grid->resolution * grid->resolution;
     occ_bits_raise_kernel<<<(n_updates + 255) / 256, 256, 0, stream>>>(n_updates, volume, grid->n_levels, density,
                                                                        bitfield, bitfield_out, levels, cells, values,
                                                                        rand_select, activation, sample_all_dev, decay,

@@ -20,6 +20,7 @@ struct tn_ctx {
     size_t block_f32_cap = 0;
     uint8_t* mip = nullptr;             // coarse occupancy mip built by tn_march_count
     size_t mip_cap = 0;
+    int* box = nullptr;                 // [BOX_INTS] occupied blocks' box, left empty by every tn_march_count
     float* slots = nullptr;             // per-ray step positions recorded by tn_march_count
     size_t slots_cap = 0;
     uint32_t slot_cap = 0;              // slots per ray of the last tn_march_count
@@ -32,6 +33,9 @@ struct tn_ctx {
 };
 
 namespace tn {
+
+constexpr int BOX_INTS = 2 * MAX_LEVELS * 3;  // per level: lo block x,y,z | hi block + 1 x,y,z
+constexpr int BOX_EMPTY_LO = 0x7F7F7F7F;      // an empty box: this | 0
 
 enum Ticket : int {
     TICKET_MARCH = 0,
@@ -127,11 +131,14 @@ int launch_occupancy_update(tn_ctx* ctx, cudaStream_t stream, const tn_grid_desc
 // The bitfield launch_occupancy_update will write into bitfield_out, computed before it from
 // settled densities without changing them (the selection rule reads `bitfield`, the policy
 // *sample_all_dev); equal to the update's bits bit for bit.
-int launch_occupancy_bits_ahead(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
-                                const uint8_t* bitfield, uint8_t* bitfield_out, uint32_t n_updates,
-                                const int32_t* levels, const uint32_t* cells, const float* values,
-                                const float* rand_select, int activation, const uint32_t* sample_all_dev, float decay,
-                                float threshold);
+// Two launches: the decayed densities' bits, then the queried cells raised (values).
+int launch_occupancy_bits_decayed(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
+                                  uint8_t* bitfield_out, float decay, float threshold);
+int launch_occupancy_bits_raised(cudaStream_t stream, const tn_grid_desc* grid, const float* density,
+                                 const uint8_t* bitfield, uint8_t* bitfield_out, uint32_t n_updates,
+                                 const int32_t* levels, const uint32_t* cells, const float* values,
+                                 const float* rand_select, int activation, const uint32_t* sample_all_dev, float decay,
+                                 float threshold);
 int launch_occupancy_scatter(cudaStream_t stream, const tn_grid_desc* grid, float* density, const uint8_t* bitfield,
                              uint32_t n_updates, const int32_t* levels, const uint32_t* cells, const float* values,
                              const float* rand_select, int activation, int sample_all, float decay);

@@ -137,7 +137,7 @@ struct tn_trainer {
     cudaStream_t stream = nullptr;
     // the occupancy query and update beside the training chain, and the next step's head
     cudaStream_t aux = nullptr, cstream = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_emit = nullptr, ev_occ = nullptr, ev_occ_all = nullptr, ev_head = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_losses = nullptr, ev_occ = nullptr, ev_occ_all = nullptr, ev_head = nullptr;
     RaySet set[2];
     int cur = 0;               // set of the last completed step (the aliases below point into it)
     bool spec_own = false;     // set cur ^ 1 holds the head of the next step, computed from own rays
@@ -260,18 +260,26 @@ static int enqueue_own_rays(tn_trainer* tr, cudaStream_t s, RaySet& q) {
                              q.target, q.bg, q.ray_t, q.ray_tmax, q.alive);
 }
 
-// Occupancy query of one step (the step keyed by *key): random cells, their sample points, the
-// density network, into set q's query buffers.
-static int enqueue_occupancy_query(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, RaySet& q,
-                                   const uint32_t* key) {
-    const tn_trainer_desc& d = tr->d;
-    int st = launch_synth_cells(s, tr->M, d.seed, key, grid.n_levels, tr->V, q.occ_levels, q.occ_cells, q.occ_rand3,
+// Occupancy query of one step (the step keyed by *key): random cells and their sample points, then
+// the density network, into set q's query buffers.
+static int enqueue_query_points(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, RaySet& q,
+                                const uint32_t* key) {
+    int st = launch_synth_cells(s, tr->M, tr->d.seed, key, grid.n_levels, tr->V, q.occ_levels, q.occ_cells, q.occ_rand3,
                                 tr->M, q.occ_rsel);
     if (st == TN_OK)
         st = tn_occupancy_sample_points(s, &grid, tr->M, q.occ_levels, q.occ_cells, q.occ_rand3, tr->M,
                                         1.0f / tr->aabb, q.occ_pos, tr->M);
-    if (st == TN_OK) st = tr->net.density(tr->net.user, s, tr->M, nullptr, tr->M, q.occ_pos, q.occ_values);
     return st;
+}
+
+static int enqueue_query_density(tn_trainer* tr, cudaStream_t s, RaySet& q) {
+    return tr->net.density(tr->net.user, s, tr->M, nullptr, tr->M, q.occ_pos, q.occ_values);
+}
+
+static int enqueue_occupancy_query(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, RaySet& q,
+                                   const uint32_t* key) {
+    const int st = enqueue_query_points(tr, s, grid, q, key);
+    return st == TN_OK ? enqueue_query_density(tr, s, q) : st;
 }
 
 // Occupancy update of the step in set pi: decay + max-update of the queried cells (the selection
@@ -290,16 +298,21 @@ static int enqueue_occupancy_update(tn_trainer* tr, cudaStream_t s, const tn_gri
                                    tr->tail_bits(pi), bits_done, bits_ready);
 }
 
-// The bitfield the occupancy update of the step in set qi will write, from its query (already in
-// set qi) and the settled densities, into the step's output bitfield; the step's selection
-// policy is the state's next_sample_all (the running step's step_begin has run, the step's has
-// not). Nothing changes the densities or the query before that update runs.
-static int enqueue_occupancy_bits_ahead(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, int qi) {
-    const tn_trainer_desc& d = tr->d;
+// The bitfield the occupancy update of the step in set qi will write, from the settled densities
+// and its query, into the step's output bitfield, in two parts: the decayed densities' bits, then
+// the queried cells raised; the step's selection policy is the state's next_sample_all (the running
+// step's step_begin has run, the step's has not). Nothing changes the densities or the query
+// before that update runs.
+static int enqueue_bits_decayed(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, int qi) {
+    return launch_occupancy_bits_decayed(s, &grid, tr->density, tr->tail_bits(qi), tr->d.occupancy_decay,
+                                         tr->d.occupancy_threshold);
+}
+
+static int enqueue_bits_raised(tn_trainer* tr, cudaStream_t s, const tn_grid_desc& grid, int qi) {
     RaySet& q = tr->set[qi];
-    return launch_occupancy_bits_ahead(s, &grid, tr->density, tr->head_bits(qi), tr->tail_bits(qi), tr->M,
-                                       q.occ_levels, q.occ_cells, q.occ_values, q.occ_rsel, tr->net.activation,
-                                       &tr->state->next_sample_all, d.occupancy_decay, d.occupancy_threshold);
+    return launch_occupancy_bits_raised(s, &grid, tr->density, tr->head_bits(qi), tr->tail_bits(qi), tr->M,
+                                        q.occ_levels, q.occ_cells, q.occ_values, q.occ_rsel, tr->net.activation,
+                                        &tr->state->next_sample_all, tr->d.occupancy_decay, tr->d.occupancy_threshold);
 }
 
 // Head of a step: its rays (own, or the caller's already in set q, clipped to the box) and the
@@ -331,10 +344,11 @@ static int enqueue_head(tn_trainer* tr, cudaStream_t s, bool external, int qi) {
 // the one the count used (or only the densities, when the bitfield was computed ahead). With
 // next >= 0 the head of the following step (rays from next_external / own rays) runs on the
 // third stream into set next, its count once the output bitfield is there, Adam keeps to
-// side_sms SMs beside it, and the following step's occupancy query runs after Adam (the
-// density network reads the updated parameters), followed by the bitfield its update will
-// write. ring >= 0 copies the finished step's state into that pinned slot before the head is
-// joined.
+// side_sms SMs beside it, and the following step's occupancy query and the bitfield its update
+// will write are made: points and decayed bits on the second stream beside Adam, the density
+// network (which reads the updated parameters) and the raised bits after it: 10 us of the tail
+// after Adam instead of 33 (the step 0.6 to 1%: the count beside it takes nearly as long). ring >= 0
+// copies the finished step's state into that pinned slot before the head is joined.
 static int enqueue_tail(tn_trainer* tr, int pi, int next, bool next_external, int ring) {
     const tn_trainer_desc& d = tr->d;
     cudaStream_t s = tr->stream, so = tr->aux, cs = tr->cstream;
@@ -352,7 +366,6 @@ static int enqueue_tail(tn_trainer* tr, int pi, int next, bool next_external, in
         st = cuda_status(cudaStreamWaitEvent(so, tr->ev_fork, 0), "fork");
         if (st == TN_OK)
             st = enqueue_occupancy_update(tr, so, grid, pi, next >= 0 && !ahead ? tr->ev_occ : nullptr, ahead);
-        if (st == TN_OK) st = cuda_status(cudaEventRecord(tr->ev_occ_all, so), "occupancy done");
     }
     // the next step's head: its rays at once, its march count on the step's output bitfield
     // (ready at once when it was computed ahead)
@@ -378,6 +391,18 @@ static int enqueue_tail(tn_trainer* tr, int pi, int next, bool next_external, in
                           d.use_distortion_loss ? d.distortion_lambda : 0.0f, tr->net_density, tr->net_rgb, tr->s_dt,
                           tr->s_mnorm, tr->s_dtnorm, tr->s_t, p.target, p.bg, nullptr, tr->grad_density, tr->dl_drgb,
                           tr->state->loss_sums, false);
+    if (st == TN_OK && occ) {
+        // the following step's query points (keyed by its index: step_count after this step_begin) and
+        // decayed bits need no parameters: they run beside Adam (the emit pass, which reads the
+        // bitfield they replace, is done; beside the losses they cost those what they saved)
+        if (next >= 0) {
+            st = cuda_status(cudaEventRecord(tr->ev_losses, s), "losses done");
+            if (st == TN_OK) st = cuda_status(cudaStreamWaitEvent(so, tr->ev_losses, 0), "after the losses");
+            if (st == TN_OK) st = enqueue_query_points(tr, so, grid, tr->set[next], &tr->state->step_count);
+            if (st == TN_OK) st = enqueue_bits_decayed(tr, so, grid, next);
+        }
+        if (st == TN_OK) st = cuda_status(cudaEventRecord(tr->ev_occ_all, so), "occupancy done");
+    }
     if (st == TN_OK && tr->net.backward)
         st = tr->net.backward(tr->net.user, s, tr->B, info + 1, tr->B, tr->s_pos, tr->s_dir, tr->grad_density,
                               tr->dl_drgb, tr->g);
@@ -392,10 +417,10 @@ static int enqueue_tail(tn_trainer* tr, int pi, int next, bool next_external, in
                          tr->steps, place);
     }
     if (st == TN_OK && occ) st = cuda_status(cudaStreamWaitEvent(s, tr->ev_occ_all, 0), "occupancy joined");
-    // the following step's occupancy query, keyed by its index (step_count after this step_begin)
-    if (st == TN_OK && occ && next >= 0) st = enqueue_occupancy_query(tr, s, grid, tr->set[next], &tr->state->step_count);
-    // and the bitfield its occupancy update will write, so that the head after it need not wait
-    if (st == TN_OK && occ && next >= 0) st = enqueue_occupancy_bits_ahead(tr, s, grid, next);
+    // the rest of the following step's occupancy query and of the bitfield its update will write
+    // (so that the head after it need not wait): what reads the updated parameters
+    if (st == TN_OK && occ && next >= 0) st = enqueue_query_density(tr, s, tr->set[next]);
+    if (st == TN_OK && occ && next >= 0) st = enqueue_bits_raised(tr, s, grid, next);
     if (st == TN_OK) {
         step_end_kernel<<<1, 1, 0, s>>>(tr->state, info, p.ctx->flags);
         st = check_launch("step_end");
@@ -752,7 +777,7 @@ int tn_trainer_create(tn_trainer** out, const tn_trainer_desc* desc, const tn_ne
     if (st == TN_OK) st = cuda_status(cudaStreamCreateWithFlags(&tr->aux, cudaStreamNonBlocking), "aux stream");
     if (st == TN_OK) st = cuda_status(cudaStreamCreateWithFlags(&tr->cstream, cudaStreamNonBlocking), "head stream");
     if (st == TN_OK) st = cuda_status(cudaStreamCreateWithFlags(&tr->h2d, cudaStreamNonBlocking), "copy stream");
-    for (cudaEvent_t* e : {&tr->ev_fork, &tr->ev_emit, &tr->ev_occ, &tr->ev_occ_all, &tr->ev_head,
+    for (cudaEvent_t* e : {&tr->ev_fork, &tr->ev_losses, &tr->ev_occ, &tr->ev_occ_all, &tr->ev_head,
                            &tr->ev_staged[0], &tr->ev_staged[1]})
         if (st == TN_OK) st = cuda_status(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "step events");
     for (int k = 0; k < 2 && st == TN_OK; ++k) st = tn_ctx_create(&tr->set[k].ctx);
@@ -847,7 +872,7 @@ int tn_trainer_destroy(tn_trainer* tr) {
     for (int k = 0; k < 2; ++k)
         if (tr->set[k].ctx) tn_ctx_destroy(tr->set[k].ctx);
     if (tr->h2d) cudaStreamSynchronize(tr->h2d);
-    for (cudaEvent_t e : {tr->ev_fork, tr->ev_emit, tr->ev_occ, tr->ev_occ_all, tr->ev_head,
+    for (cudaEvent_t e : {tr->ev_fork, tr->ev_losses, tr->ev_occ, tr->ev_occ_all, tr->ev_head,
                           tr->ev_staged[0], tr->ev_staged[1]})
         if (e) cudaEventDestroy(e);
     if (tr->h2d) cudaStreamDestroy(tr->h2d);
