@@ -78,21 +78,23 @@ class DistortionLoss(torch.autograd.Function):
         offsets = _check(offsets, "offsets", torch.int32)
         S, R = sigma.numel(), counts.numel()
         rb = hp.ray_batch(counts, offsets, R, R, S)
-        out = hp.distortion_fwd_bwd(_ctx(sigma.device), rb, sigma, m_norm, dt_norm, lam, activation=activation,
-                                    backward=False)
+        ray_loss = torch.zeros(R, dtype=torch.float32, device=sigma.device)
+        hp.distortion_call(_ctx(sigma.device), rb, sigma, m_norm, dt_norm, lam, activation, None, ray_loss, None,
+                           None)
         ctx.save_for_backward(sigma, m_norm, dt_norm, counts, offsets)
         ctx.lam = lam
         ctx.activation = activation
-        return out["ray_loss"]
+        return ray_loss
 
     @staticmethod
     def backward(ctx, grad_ray):
         sigma, m_norm, dt_norm, counts, offsets = ctx.saved_tensors
         S, R = sigma.numel(), counts.numel()
         rb = hp.ray_batch(counts, offsets, R, R, S)
-        out = hp.distortion_fwd_bwd(_ctx(sigma.device), rb, sigma, m_norm, dt_norm, ctx.lam,
-                                    activation=ctx.activation, grad_ray=grad_ray.contiguous().to(torch.float32))
-        return out["dL_ddensity"], None, None, None, None, None, None
+        dd = torch.zeros(S, dtype=torch.float32, device=sigma.device)
+        hp.distortion_call(_ctx(sigma.device), rb, sigma, m_norm, dt_norm, ctx.lam, ctx.activation,
+                           grad_ray.contiguous().to(torch.float32), None, None, dd)
+        return dd, None, None, None, None, None, None
 
 
 def composite(sigma, rgb, dt, counts, offsets, min_transmittance=1e-4, activation=0):

@@ -440,8 +440,8 @@ __device__ __forceinline__ uint2 balanced_rays(const uint32_t* __restrict__ coun
 
 // ---- kernels ----------------------------------------------------------------------------
 // ---- sample tiles over several rays (the compositor's launch form) -------------------------
-// Each warp owns a run of consecutive rays (`rpw` of them in the distortion tiles; the rays that
-// start in its share of the samples in the compositor tiles, balanced_rays), whose samples are one
+// Each warp owns a run of consecutive rays (those that start in its share of the samples,
+// balanced_rays), whose samples are one
 // contiguous range (offsets are the exclusive scan of the counts), and walks that range in tiles
 // of 32 * K samples, lane l owning
 // the K consecutive samples [base + K l, base + K l + K). Short rays share a tile and long rays
@@ -515,6 +515,28 @@ __device__ __forceinline__ void seg_scan_plan(float (&v)[N], uint32_t plan) {
         for (int k = 0; k < N; ++k) {
             const float vo = SUFFIX ? __shfl_down_sync(FULL_MASK, v[k], d) : __shfl_up_sync(FULL_MASK, v[k], d);
             if ((plan >> l) & 1u) v[k] += vo;
+        }
+    }
+}
+
+// The plan as a distance read off one ballot instead of five shuffles: lanes up to that far below
+// (above, SUFFIX) belong to this lane's segment, so a level adds when its distance is no larger.
+// The same additions. The distortion tiles take this form (gradient launch 97.5 -> 89.6 us on 2^22
+// samples); the compositor's VJP is 35.4 us with seg_plan and 36.8 with this one.
+template <bool SUFFIX>
+__device__ __forceinline__ int seg_reach(bool cut, int lane) {
+    const uint32_t cuts = __ballot_sync(FULL_MASK, cut);
+    return SUFFIX ? __ffs((int)((cuts | 0x80000000u) >> lane)) - 1 : __clz((int)((cuts | 1u) << (WARP - 1 - lane)));
+}
+
+template <int N, bool SUFFIX>
+__device__ __forceinline__ void seg_scan_reach(float (&v)[N], int reach) {
+#pragma unroll
+    for (int d = 1; d < WARP; d *= 2) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const float vo = SUFFIX ? __shfl_down_sync(FULL_MASK, v[k], d) : __shfl_up_sync(FULL_MASK, v[k], d);
+            if (reach >= d) v[k] += vo;
         }
     }
 }
@@ -1061,7 +1083,8 @@ composite_bwd_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, ui
 // ---- distortion loss over sample tiles ------------------------------------------------------
 // The distortion loss forward and backward (mipNeRF360_distortion_loss_forward_kernel /
 // _backward_kernel, training-kernels-fused.cuh:13-224, with the sums A, B above) in the tile
-// form of the compositor: a warp owns `rpw` consecutive rays and walks their samples in tiles of
+// form of the compositor: a warp takes the rays that start in its share of the samples
+// (balanced_rays), in groups of at most `group`, and walks a group's samples in tiles of
 // 32 * K, lane l owning K consecutive samples. Forward, tiles in increasing order: per sample the
 // optical depth before it, the weight w = T (1 - e^-x), the weight sum before it W_<, the
 // increment dm of m and A = sum dm W_<, each a segmented scan of the lane aggregates with a
@@ -1072,6 +1095,15 @@ composite_bwd_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, ui
 // suffix sums W_>=, F = sum dm W_>= (B = F of the next sample) and sum g w over later samples,
 // with g = k ((2/3) dtn w + 2 (A + B)) and dL/dsigma = dtn (g T_{j+1} - sum_{l>j} g_l w_l).
 // Tiles past the kept ones replay the forward from the last kept carry.
+// A launch that only wants the gradient leaves the loss sums out, and the forward of each group's
+// last tile, whose carry nobody reads.
+// Bound by instruction issue (dependent scans, 24 warps an SM), not by its 12 or 16 bytes a sample
+// (8 and 11 us at 2^22 samples). The shares are of samples: with the same number of rays a warp,
+// one wave ended with the warp whose rays happened to be long (geometric lengths, 19 rays a warp:
+// 1.5 to 1.8 times the mean). Loss launch and gradient launch, mean 64 samples a ray, 2^22 samples:
+// 46.2 and 108.8 us before, 38.0 and 69.9 now; 5e5 samples, mean 128: 22.8 and 57.7, 20.2 and 41.2;
+// 4e6, mean 5: 66.9 and 123.6, 57.2 and 84.0; 6e4, mean 20: 9.0 and 16.0, 6.6 and 11.6. Loss of 5e5
+// samples, mean 6: 10.7, 11.7 now (the search for the shares), its gradient 21.4, 16.5.
 
 struct DistTile {
     float sig[ST_K], dtn[ST_K], w[ST_K], tn[ST_K], dm[ST_K], a[ST_K];
@@ -1081,7 +1113,7 @@ struct DistTile {
 // carry at its end.
 template <bool VEC, int ACT>
 __device__ __forceinline__ void dist_tile_forward(const Samples& S, uint32_t s0, const bool (&in)[ST_K],
-                                                  const bool (&head)[ST_K], bool any_head, uint32_t plan, int lane,
+                                                  const bool (&head)[ST_K], bool any_head, int reach, int lane,
                                                   const DistCarry& c, DistCarry& next, DistTile& d) {
     constexpr int K = ST_K;
     float m[K];
@@ -1123,7 +1155,7 @@ __device__ __forceinline__ void dist_tile_forward(const Samples& S, uint32_t s0,
         agg[0] += x[q];
     }
     if (lane == 0 && !any_head) agg[0] += c.x;
-    seg_scan_plan<1, false>(agg, plan);
+    seg_scan_reach<1, false>(agg, reach);
     float run = shift_up(agg[0], lane, c.x);
     // T before the lane's first sample; inside a ray the transmittance before a sample is the one
     // after the previous sample, the same exp of the same depth. After a sample it is exp(-depth),
@@ -1147,7 +1179,7 @@ __device__ __forceinline__ void dist_tile_forward(const Samples& S, uint32_t s0,
         agg[0] += d.w[q];
     }
     if (lane == 0 && !any_head) agg[0] += c.w;
-    seg_scan_plan<1, false>(agg, plan);
+    seg_scan_reach<1, false>(agg, reach);
     run = shift_up(agg[0], lane, c.w);
 #pragma unroll
     for (int q = 0; q < K; ++q) {
@@ -1166,7 +1198,7 @@ __device__ __forceinline__ void dist_tile_forward(const Samples& S, uint32_t s0,
         agg[0] += d.dm[q] * wex[q];
     }
     if (lane == 0 && !any_head) agg[0] += c.a;
-    seg_scan_plan<1, false>(agg, plan);
+    seg_scan_reach<1, false>(agg, reach);
     run = shift_up(agg[0], lane, c.a);
 #pragma unroll
     for (int q = 0; q < K; ++q) {
@@ -1201,7 +1233,7 @@ __device__ __forceinline__ void tile_flags(const uint32_t* t_off, const uint32_t
 
 template <bool VEC, int ACT>
 __global__ void __launch_bounds__(LOSS_THREADS)
-distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint32_t rpw,
+distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint32_t group,
                         const uint32_t* __restrict__ counts, const uint32_t* __restrict__ offsets, float lambda,
                         const float* __restrict__ grad_ray, float* __restrict__ ray_loss, float* loss_sum,
                         float* __restrict__ dd, float* partials, uint32_t* ticket) {
@@ -1210,10 +1242,12 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
     __shared__ float t_k[LOSS_WARPS][WARP], t_gs[LOSS_WARPS][WARP];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_live = live_rays(n_rays, n_dev);
-    const uint32_t r0 = (blockIdx.x * LOSS_WARPS + wid) * rpw;
+    uint2 rr = make_uint2(0u, 0u);
+    if (n_live) rr = balanced_rays(counts, offsets, n_live, blockIdx.x * LOSS_WARPS + wid, gridDim.x * LOSS_WARPS, lane);
     float acc[1] = {0.0f};
-    if (r0 < n_live) {  // whole warps; every thread reaches the block sum below
-        const int nr = (int)min(rpw, n_live - r0);
+    for (uint32_t r0 = rr.x; r0 < rr.y; r0 += group) {  // whole warps; every thread reaches the block sum below
+        const int nr = (int)min(group, rr.y - r0);
+        __syncwarp();  // the group before has read its tables
         if (lane < nr) {
             const uint32_t r = r0 + lane, o = offsets[r], n = counts[r];
             t_off[wid][lane] = o;
@@ -1230,11 +1264,14 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
         // forward: carries kept for the backward (tile t in lane t % 32, slot t / 32)
         DistCarry keep0{0.0f, 0.0f, 0.0f, 0.0f}, keep1 = keep0;
         DistCarry c{0.0f, 0.0f, 0.0f, 0.0f};
+        const bool want_loss = ray_loss != nullptr || loss_sum != nullptr;
         float cl[2] = {0.0f, 0.0f};  // running loss sums (sum dtn w^2, sum w A) of the open ray
         for (uint32_t t = 0; t < n_tiles; ++t) {
             if ((uint32_t)lane == (t & 31u)) {
                 if (t < 32u) keep0 = c; else if (t < 64u) keep1 = c;
             }
+            // without the loss only the carries are wanted, and the last tile's leads nowhere
+            if (!want_loss && t + 1 == n_tiles) break;
             const uint32_t s0 = b0 + t * span + (uint32_t)lane * K;
             bool in[K], head[K], last[K];
             int ri[K];
@@ -1242,10 +1279,12 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
             bool any_head = false;
 #pragma unroll
             for (int q = 0; q < K; ++q) any_head = any_head || head[q];
-            const uint32_t plan = seg_plan<false>(any_head, lane);
+            const int reach = seg_reach<false>(any_head, lane);
             DistTile d;
             DistCarry nx;
-            dist_tile_forward<VEC, ACT>(S, s0, in, head, any_head, plan, lane, c, nx, d);
+            dist_tile_forward<VEC, ACT>(S, s0, in, head, any_head, reach, lane, c, nx, d);
+            c = nx;
+            if (!want_loss) continue;
             float l2[2] = {0.0f, 0.0f};
 #pragma unroll
             for (int q = 0; q < K; ++q) {
@@ -1254,7 +1293,7 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                 l2[1] += d.w[q] * d.a[q];
             }
             if (lane == 0 && !any_head) { l2[0] += cl[0]; l2[1] += cl[1]; }
-            seg_scan_plan<2, false>(l2, plan);
+            seg_scan_reach<2, false>(l2, reach);
             float e2[2] = {shift_up(l2[0], lane, cl[0]), shift_up(l2[1], lane, cl[1])};
 #pragma unroll
             for (int q = 0; q < K; ++q) {
@@ -1269,7 +1308,6 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
             }
             cl[0] = __shfl_sync(FULL_MASK, l2[0], WARP - 1);
             cl[1] = __shfl_sync(FULL_MASK, l2[1], WARP - 1);
-            c = nx;
         }
         if (dd) {
             // backward: tiles from the last; suffix carries of the ray open at each tile's end
@@ -1299,7 +1337,7 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                         for (int q = 0; q < K; ++q) any_head = any_head || head[q];
                         DistTile du;
                         DistCarry nx;
-                        dist_tile_forward<VEC, ACT>(S, su, in, head, any_head, seg_plan<false>(any_head, lane), lane,
+                        dist_tile_forward<VEC, ACT>(S, su, in, head, any_head, seg_reach<false>(any_head, lane), lane,
                                                     ct, nx, du);
                         ct = nx;
                     }
@@ -1316,9 +1354,9 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                 }
                 DistTile d;
                 DistCarry nx;
-                dist_tile_forward<VEC, ACT>(S, s0, in, head, any_head, seg_plan<false>(any_head, lane), lane, ct, nx,
+                dist_tile_forward<VEC, ACT>(S, s0, in, head, any_head, seg_reach<false>(any_head, lane), lane, ct, nx,
                                             d);
-                const uint32_t splan = seg_plan<true>(any_tail, lane);
+                const int sreach = seg_reach<true>(any_tail, lane);
                 // W_>= (inclusive suffix of w)
                 float agg[1] = {0.0f};
 #pragma unroll
@@ -1327,7 +1365,7 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                     agg[0] += d.w[q];
                 }
                 if (lane == WARP - 1 && !any_tail) agg[0] += sw;
-                seg_scan_plan<1, true>(agg, splan);
+                seg_scan_reach<1, true>(agg, sreach);
                 float run = shift_down(agg[0], lane, sw);
                 float wge[K];
 #pragma unroll
@@ -1344,7 +1382,7 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                     agg[0] += d.dm[q] * wge[q];
                 }
                 if (lane == WARP - 1 && !any_tail) agg[0] += sf;
-                seg_scan_plan<1, true>(agg, splan);
+                seg_scan_reach<1, true>(agg, sreach);
                 run = shift_down(agg[0], lane, sf);
                 float g[K];
 #pragma unroll
@@ -1362,7 +1400,7 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
                     agg[0] += g[q] * d.w[q];
                 }
                 if (lane == WARP - 1 && !any_tail) agg[0] += sg;
-                seg_scan_plan<1, true>(agg, splan);
+                seg_scan_reach<1, true>(agg, sreach);
                 run = shift_down(agg[0], lane, sg);
                 float o[K];
 #pragma unroll
@@ -2571,29 +2609,21 @@ static int launch_train_losses(tn_ctx* ctx, cudaStream_t stream, const tn_ray_ba
                                            target, bg, ray_rgba, grad_density, drgb, loss_sums, accumulate);
 }
 
-// Rays per warp of the sample-tile kernels, from the batch's mean samples per ray
-// (sample_stride / n_rays, an upper bound): up to 4 tiles (32 * ST_K samples each) of samples per
-// warp while that leaves at least 32 warps per SM (the setup of a warp's range and its partly
-// filled first and last tiles are then paid once per 4 tiles), else 1 tile per warp; more when
-// the grid would otherwise take more than one wave of resident warps.
-static uint32_t tile_rays_per_warp(const tn_ray_batch* b, const void* kernel, uint32_t max_tiles = 0,
-                                   int k = ST_K) {
+// Blocks of the distortion tiles: by the batch's mean samples per ray (sample_stride / n_rays, an
+// upper bound) about one tile (32 * ST_K samples) a warp while that leaves warps per SM idle, up
+// to 4 when it does not (the setup of a warp's range and its partly filled first and last tiles
+// are then paid once per 4 tiles), and at most one wave of resident warps. `group`: rays of at
+// most 32 tiles on average, half of those whose carries a warp keeps.
+static int distortion_grid(const tn_ray_batch* b, const void* kernel, uint32_t& group) {
     const double mean = b->n_rays ? std::max(1.0, (double)b->sample_stride / (double)b->n_rays) : 1.0;
-    const double per_tile = (double)(WARP * k);
+    const double per_tile = (double)(WARP * ST_K);
     const double fill = (double)b->sample_stride / (per_tile * num_sms() * 32.0);
     const double tiles = std::min(4.0, std::max(1.0, std::floor(fill)));
-    uint32_t rpw = (uint32_t)std::min(32.0, std::max(1.0, std::floor(tiles * per_tile / mean)));
-    // when the grid would take more than one wave of resident warps, enough rays per warp (at most
-    // 32) that it takes one: no partly filled last wave
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, LOSS_THREADS, 0) == cudaSuccess && per_sm > 0) {
-        const uint64_t resident = (uint64_t)num_sms() * (uint64_t)per_sm * LOSS_WARPS;
-        const uint64_t warps = (b->n_rays + rpw - 1) / rpw;
-        if (warps > resident) rpw = (uint32_t)std::min<uint64_t>(32, (b->n_rays + resident - 1) / resident);
-    }
-    // a kernel that keeps per-tile state for max_tiles tiles: rays of about that many tiles a warp
-    if (max_tiles) rpw = std::min(rpw, (uint32_t)std::max(1.0, std::floor(max_tiles * per_tile / mean)));
-    return rpw;
+    const uint32_t rpw = (uint32_t)std::min(32.0, std::max(1.0, std::floor(tiles * per_tile / mean)));
+    group = (uint32_t)std::min(32.0, std::max(1.0, std::floor(SAVED_TILES / 2 * per_tile / mean)));
+    const uint32_t wave = (uint32_t)num_sms() * (uint32_t)blocks_per_sm(kernel, LOSS_THREADS);
+    const uint32_t warps = (b->n_rays + rpw - 1) / rpw;
+    return (int)std::min(wave, (warps + LOSS_WARPS - 1) / LOSS_WARPS);
 }
 
 // 16-byte sample vectors: every per-sample array 16-byte aligned and the stride a multiple of 4.
@@ -2604,17 +2634,9 @@ static bool tile_vec(const Samples& S, const void* a, const void* b) {
 
 // One wave of resident warps for a sample-balanced launch, at least eight rays a warp on average.
 static int balanced_grid(uint32_t n_rays, const void* kernel) {
-    int per_sm = 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, LOSS_THREADS, 0) != cudaSuccess || per_sm < 1)
-        per_sm = 1;
-    const uint32_t wave = (uint32_t)num_sms() * (uint32_t)per_sm;
+    const uint32_t wave = (uint32_t)num_sms() * (uint32_t)blocks_per_sm(kernel, LOSS_THREADS);
     const uint32_t want = (std::max(1u, n_rays / 8u) + LOSS_WARPS - 1) / LOSS_WARPS;
     return (int)std::max(1u, std::min(wave, want));
-}
-
-static int tile_grid(uint32_t n_rays, uint32_t rpw) {
-    const uint32_t warps = (n_rays + rpw - 1) / rpw;
-    return (int)((warps + LOSS_WARPS - 1) / LOSS_WARPS);
 }
 
 // Launch of the compositor forward tiles, specialised on the vector loads, the activation and
@@ -2801,15 +2823,15 @@ int tn_distortion_fwd_bwd(tn_ctx* ctx, tn_stream_t stream, const tn_ray_batch* b
     Samples S{density, nullptr, nullptr, m_norm, dt_norm, nullptr, batch->sample_stride, activation};
     const uintptr_t al = (uintptr_t)density | (uintptr_t)m_norm | (uintptr_t)dt_norm | (uintptr_t)dL_ddensity;
     const bool vec = (al & 15u) == 0 && (batch->sample_stride & 3u) == 0;
-    const uint32_t rpw = tile_rays_per_warp(
+    uint32_t group;
+    const int grid = distortion_grid(
         batch, vec ? (const void*)distortion_tiles_kernel<true, 0> : (const void*)distortion_tiles_kernel<false, 0>,
-        SAVED_TILES / 2);
-    const int grid = tile_grid(batch->n_rays, rpw);
+        group);
     st = ensure_block_f32(ctx, (size_t)grid * 2);
     if (st != TN_OK) return st;
 #define TN_DIST_TILES(V, A)                                                                                     \
     distortion_tiles_kernel<V, A><<<grid, LOSS_THREADS, 0, stream>>>(                                           \
-        S, batch->n_rays, batch->n_rays_dev, rpw, batch->counts, batch->offsets, lambda, grad_ray, ray_loss,     \
+        S, batch->n_rays, batch->n_rays_dev, group, batch->counts, batch->offsets, lambda, grad_ray, ray_loss,   \
         loss_sum, dL_ddensity, ctx->block_f32, ctx->tickets + TICKET_DIST)
     switch ((vec ? 2 : 0) | (activation ? 1 : 0)) {
         case 0: TN_DIST_TILES(false, 0); break;

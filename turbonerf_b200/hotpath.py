@@ -405,15 +405,21 @@ def recon_loss_fwd_bwd(ctx, rb: RayBatchDesc, density, rgb, dt, target_rgba, bg_
     return out
 
 
+def distortion_call(ctx, rb: RayBatchDesc, density, m_norm, dt_norm, lam, activation, grad_ray, ray_loss, loss_sum,
+                    dL_ddensity):
+    """tn_distortion_fwd_bwd into the caller's buffers; an output that is None is left out."""
+    call("tn_distortion_fwd_bwd", ctx.handle, _stream(), ctypes.byref(rb), activation, lam, _ptr(density),
+         _ptr(m_norm), _ptr(dt_norm), _ptr(grad_ray), _ptr(ray_loss), _ptr(loss_sum), _ptr(dL_ddensity))
+
+
 def distortion_fwd_bwd(ctx, rb: RayBatchDesc, density, m_norm, dt_norm, lam, activation=0, grad_ray=None,
                        backward=True):
     dev = density.device
     out = dict(ray_loss=torch.zeros(rb.ray_stride, dtype=torch.float32, device=dev),
                loss_sum=torch.zeros(1, dtype=torch.float32, device=dev),
                dL_ddensity=torch.zeros(rb.sample_stride, dtype=torch.float32, device=dev) if backward else None)
-    call("tn_distortion_fwd_bwd", ctx.handle, _stream(), ctypes.byref(rb), activation, lam, _ptr(density),
-         _ptr(m_norm), _ptr(dt_norm), _ptr(grad_ray), _ptr(out["ray_loss"]), _ptr(out["loss_sum"]),
-         _ptr(out["dL_ddensity"]))
+    distortion_call(ctx, rb, density, m_norm, dt_norm, lam, activation, grad_ray, out["ray_loss"], out["loss_sum"],
+                    out["dL_ddensity"])
     return out
 
 
