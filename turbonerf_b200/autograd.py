@@ -78,7 +78,7 @@ class DistortionLoss(torch.autograd.Function):
         offsets = _check(offsets, "offsets", torch.int32)
         S, R = sigma.numel(), counts.numel()
         rb = hp.ray_batch(counts, offsets, R, R, S)
-        ray_loss = torch.zeros(R, dtype=torch.float32, device=sigma.device)
+        ray_loss = torch.empty(R, dtype=torch.float32, device=sigma.device)
         hp.distortion_call(_ctx(sigma.device), rb, sigma, m_norm, dt_norm, lam, activation, None, ray_loss, None,
                            None)
         ctx.save_for_backward(sigma, m_norm, dt_norm, counts, offsets)

@@ -722,12 +722,13 @@ __device__ __forceinline__ void composite_fwd_group(const Samples& S, uint32_t r
     if (lane < nr) {
         o = offsets[r0 + lane];
         c = counts[r0 + lane];
-        if (c == 0) {  // a ray without samples
-            const uint32_t r = r0 + lane;
-            rgba[r] = 0.0f; rgba[r + rs] = 0.0f; rgba[r + 2 * (size_t)rs] = 0.0f; rgba[r + 3 * (size_t)rs] = 0.0f;
-            if (depth) depth[r] = 0.0f;
-            if (n_used) n_used[r] = 0u;
-        }
+        // Every ray starts out empty: the final state of one without samples, and what a ray keeps
+        // whose depth is no number (it never terminates). So callers pass buffers as allocated: a
+        // fill costs the host 7 to 11 us, this 24 bytes a ray. The sync below orders the stores.
+        const uint32_t r = r0 + lane;
+        rgba[r] = 0.0f; rgba[r + rs] = 0.0f; rgba[r + 2 * (size_t)rs] = 0.0f; rgba[r + 3 * (size_t)rs] = 0.0f;
+        if (depth) depth[r] = 0.0f;
+        if (n_used) n_used[r] = 0u;
     }
     const unsigned ne = __ballot_sync(FULL_MASK, c > 0u);
     if (ne == 0u) return;

@@ -22,11 +22,15 @@ def _ptr(t):
         raise ValueError("turbo_hot tensors must live on a CUDA device")
     if not t.is_contiguous():
         raise ValueError("turbo_hot tensors must be contiguous")
-    return ctypes.c_void_p(t.data_ptr())
+    return t.data_ptr()  # the C signatures turn the integer into a pointer
 
 
 def _stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    """torch's current stream as an address, without the torch.cuda.Stream object around it (3.4 us
+    of host time a call); where torch has not initialised CUDA yet, that object does."""
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 class Context:
@@ -117,9 +121,11 @@ def ray_batch(counts: torch.Tensor, offsets: torch.Tensor, n_rays: int, ray_stri
 # ---- rays -------------------------------------------------------------------------------
 def rays_init_bbox(ori, dir_, n_rays, ray_stride, bbox, t_far=3.0e38):
     dev = ori.device
-    t = torch.zeros(ray_stride, dtype=torch.float32, device=dev)
-    tmax = torch.zeros(ray_stride, dtype=torch.float32, device=dev)
-    alive = torch.zeros(ray_stride, dtype=torch.uint8, device=dev)
+    # every ray is written: only entries past the last one need the zeros
+    make = torch.empty if n_rays == ray_stride else torch.zeros
+    t = make(ray_stride, dtype=torch.float32, device=dev)
+    tmax = make(ray_stride, dtype=torch.float32, device=dev)
+    alive = make(ray_stride, dtype=torch.uint8, device=dev)
     b = bbox_desc(bbox)
     call("tn_rays_init_bbox", _stream(), n_rays, ray_stride, ctypes.byref(b), t_far, _ptr(ori), _ptr(dir_), _ptr(t),
          _ptr(tmax), _ptr(alive))
@@ -341,9 +347,11 @@ def composite_fwd(ctx, rb: RayBatchDesc, density, rgb, dt, activation=0, min_t=1
     dev = density.device
     rs = rb.ray_stride
     if out is None:
-        out = dict(rgba=torch.zeros(4 * rs, dtype=torch.float32, device=dev),
-                   depth=torch.zeros(rs, dtype=torch.float32, device=dev),
-                   n_used=torch.zeros(rs, dtype=torch.int32, device=dev))
+        # every ray of the batch is written: only entries past the last one need the zeros
+        make = torch.empty if rb.n_rays == rs and not rb.n_rays_dev else torch.zeros
+        out = dict(rgba=make(4 * rs, dtype=torch.float32, device=dev),
+                   depth=make(rs, dtype=torch.float32, device=dev),
+                   n_used=make(rs, dtype=torch.int32, device=dev))
     call("tn_composite_fwd", ctx.handle, _stream(), ctypes.byref(rb), activation, min_t, _ptr(density), _ptr(rgb),
          _ptr(dt), _ptr(out["rgba"]), _ptr(out["depth"]), _ptr(out["n_used"]))
     return out
@@ -497,7 +505,8 @@ def plain_grad_epilogue(n_samples, loss_scale, dL_rec, dL_dist, t, grad_out):
 def occupancy_sample_points(grid: GridSpec, levels, cells, rand3, rand_stride, inv_aabb, pos_stride=None):
     n = levels.numel()
     pos_stride = pos_stride or n
-    out = torch.zeros(3 * pos_stride, dtype=torch.float32, device=levels.device)
+    make = torch.empty if pos_stride == n else torch.zeros  # every point is written
+    out = make(3 * pos_stride, dtype=torch.float32, device=levels.device)
     g = grid.desc()
     call("tn_occupancy_sample_points", _stream(), ctypes.byref(g), n, _ptr(levels), _ptr(cells), _ptr(rand3),
          rand_stride, inv_aabb, _ptr(out), pos_stride)
