@@ -36,6 +36,8 @@ struct RenderArgs {
     float train_size_x, train_size_y, train_size_z;  // training box extents (pos_to_unit)
     float inv_train_size;                             // 1 / training box size (its x extent)
     float cone, dt_min, dt_max;
+    float t_hold;          // up to this t every step is dt_min: t cone stays below it
+    float t_grow, t_full;  // between these every step is t cone
     float min_t;
     int act;
     // level choice from float bit patterns (valid when level k's half extent and cell size are
@@ -157,6 +159,33 @@ __device__ __forceinline__ void axis_window(float o, float d, float inv_d, float
     }
 }
 
+// Many steps t = fl(t + d) of one length d at once, exactly as the additions one by one. Between two
+// powers of two the floats are the multiples of one ulp u: t = T u, and fl(T u + d) = (T + I) u with
+// I the integer nearest to d / u, the same for every t, as long as the result stays below the next
+// power of two and d / u is not halfway between two integers (then T's parity decides). d / u is
+// exact, a scaling by a power of two. So n steps give (T + n I) u, which is the bit pattern of t plus
+// n I. n is a whole step or two less than what fits below `lim`, so that the caller's plain steps
+// decide where the stretch ends; fewer than 8 steps are left to them (the set-up costs as much).
+// The walk's first round of an 800 x 800 frame (63 untested steps a tested one) was bound by issuing
+// these steps: 636 us one by one, 532 with this, 405 with the growing steps four per end test too.
+// t advances by the n steps returned; `stop` is how far plain steps may go before it is worth asking
+// again: the stretch's end, or the end of t's power of two.
+__device__ __forceinline__ uint32_t steps_at_once(float& t, float d, float lim, uint32_t max_steps, float& stop) {
+    const uint32_t bits = __float_as_uint(t), e = bits >> 23;
+    if (e - 32u >= 200u) {  // near zero (the ray's first steps), negative or huge: one plain step
+        stop = t;
+        return 0u;
+    }
+    stop = fminf(lim, __uint_as_float(bits | 0x7FFFFFu));
+    const float per_ulp = __uint_as_float((277u - e) << 23);  // 1 / u = 2^(150 - e)
+    const float q = d * per_ulp, inc = rintf(q);
+    const float room = (stop - t) * per_ulp;  // exact: both are multiples of u, less than 2^23 apart
+    if (!(room > 8.0f * inc) || !(inc >= 1.0f) || fabsf(q - inc) == 0.5f) return 0u;
+    const uint32_t n = min((uint32_t)__fdividef(room, inc) - 1u, max_steps);
+    t = __uint_as_float(bits + n * (uint32_t)inc);
+    return n;
+}
+
 // One round of one ray: from its t, the steps t += get_dt(t) of the reference's march
 // (march_rays_and_generate_global_sample_points_kernel, rendering-kernels.cu:264-334), each sample
 // tested as filter_and_localize_samples_for_nerf_kernel and assign_normalized_network_inputs_kernel
@@ -251,20 +280,33 @@ __device__ WalkResult render_walk(const RenderArgs& A, const RayMarch& r, float 
                     const float t_in = fmaxf(ix0, fmaxf(iy0, iz0));
                     const float t_out = fminf(fminf(ix1, fminf(iy1, iz1)), tmax);
                     if (t >= t_in) {
-                        // once t cone has reached dt_max every later step is dt_max (t only grows):
-                        // four steps per window test; t is monotone, so the fourth decides
-                        if (__fmul_rn(t, A.cone) >= A.dt_max) {
-                            while (iters + 4u <= max_iters) {
-                                const float t4 = __fadd_rn(
-                                    __fadd_rn(__fadd_rn(__fadd_rn(t, A.dt_max), A.dt_max), A.dt_max), A.dt_max);
-                                if (!(t4 <= t_out)) break;
-                                t = t4;
-                                iters += 4u;
-                            }
-                        }
                         while (t <= t_out && iters < max_iters) {
-                            t = __fadd_rn(t, get_dt(t, A.cone, A.dt_min, A.dt_max));
-                            ++iters;
+                            // where the step length is constant (t cone at most dt_min, or at
+                            // least dt_max: t only grows) all but the last steps are one addition
+                            float stop = t_out;  // plain steps until t is past it
+                            const bool at_max = __fmul_rn(t, A.cone) >= A.dt_max;
+                            if (at_max || t <= A.t_hold) {
+                                const float lim = at_max ? t_out : fminf(t_out, A.t_hold);
+                                const uint32_t n = steps_at_once(t, at_max ? A.dt_max : A.dt_min, lim,
+                                                                 max_iters - iters - 1u, stop);
+                                iters += n;
+                            } else if (t >= A.t_grow) {
+                                // every step is t cone up to t_full: four per end test (t is
+                                // monotone, so the fourth decides), no clamps
+                                stop = fminf(t_out, A.t_full);
+                                while (iters + 5u <= max_iters) {
+                                    float u = t;
+#pragma unroll
+                                    for (int q = 0; q < 4; ++q) u = __fadd_rn(u, __fmul_rn(u, A.cone));
+                                    if (!(u <= stop)) break;
+                                    t = u;
+                                    iters += 4u;
+                                }
+                            }
+                            do {
+                                t = __fadd_rn(t, get_dt(t, A.cone, A.dt_min, A.dt_max));
+                                ++iters;
+                            } while (t <= stop && iters < max_iters);
                         }
                     }
                 }
@@ -522,6 +564,10 @@ int tn_render(tn_ctx* ctx, tn_stream_t stream, const tn_render_desc* desc, const
     A.cone = desc->cone_angle;
     A.dt_min = desc->dt_min;
     A.dt_max = 8.0f * desc->dt_min;  // renderer.cu:305
+    // a hair inside the exact bounds, so that no rounding of t cone reaches the other side
+    A.t_hold = A.cone > 0.0f ? A.dt_min / A.cone * (1.0f - 1e-6f) : INFINITY;
+    A.t_grow = A.cone > 0.0f ? A.dt_min / A.cone * (1.0f + 1e-6f) : INFINITY;
+    A.t_full = A.cone > 0.0f ? A.dt_max / A.cone * (1.0f - 1e-6f) : INFINITY;
     A.min_t = desc->min_transmittance;
     A.act = net->activation;
     {
