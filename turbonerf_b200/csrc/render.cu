@@ -166,7 +166,7 @@ __device__ __forceinline__ void axis_window(float o, float d, float inv_d, float
 // exact, a scaling by a power of two. So n steps give (T + n I) u, which is the bit pattern of t plus
 // n I. n is a whole step or two less than what fits below `lim`, so that the caller's plain steps
 // decide where the stretch ends; fewer than 8 steps are left to them (the set-up costs as much).
-// The walk's first round of an 800 x 800 frame (63 untested steps a tested one) was bound by issuing
+// The walk's first round of an 800 x 800 frame (about 30 untested steps a tested one) was bound by issuing
 // these steps: 636 us one by one, 532 with this, 405 with the growing steps four per end test too.
 // t advances by the n steps returned; `stop` is how far plain steps may go before it is worth asking
 // again: the stretch's end, or the end of t's power of two.
