@@ -644,7 +644,7 @@ __device__ __forceinline__ uint32_t count_ray(const MarchArgs& a, const CountGri
 // occupied 4x4x4 blocks padded by one cell of that level; points beyond the grid clamp to the
 // coarsest level's edge cells, so an occupied edge block of that level opens its side to
 // infinity. cut = 2 when no cell is occupied.
-__device__ void occupied_union(const CountGrid& cg, const int* __restrict__ box, int n_levels, float* u, int* cut) {
+__device__ void occupied_union(const CountGrid& cg, const int* box, int n_levels, float* u, int* cut) {
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     const int C = 1 << (cg.res_shift - 2);
     bool any = false;
@@ -767,6 +767,9 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
     scan_blocks_and_cut<COUNT_GROUP_MAX>(gridDim.x, n_live, counts, block_agg, block_prefix, batch_size, batch_info,
                                      flags);
     if (threadIdx.x == 0) *ticket = 0u;
+    // every block read the box before it took its ticket: the next call's build starts from an empty one
+    if (MIP)
+        for (int k = threadIdx.x; k < BOX_INTS; k += blockDim.x) box_g[k] = k < BOX_INTS / 2 ? BOX_EMPTY_LO : 0;
 }
 
 constexpr int EXPAND_U = 4;
@@ -1461,6 +1464,11 @@ static int launch_count(uint32_t nb, uint32_t group, size_t smem, cudaStream_t s
     return check_launch("tn_march_count");
 }
 
+static void empty_box(tn_ctx* ctx, cudaStream_t stream) {
+    cudaMemsetAsync(ctx->box, BOX_EMPTY_LO & 0xFF, BOX_INTS / 2 * sizeof(int), stream);
+    cudaMemsetAsync(ctx->box + BOX_INTS / 2, 0, BOX_INTS / 2 * sizeof(int), stream);
+}
+
 // The two passes of the compaction with a tile of BLOCK x ITEMS values.
 template <int BLOCK, int ITEMS>
 static void launch_compact(cudaStream_t stream, uint32_t nb, uint32_t n, const uint32_t* values, tn_ctx* ctx,
@@ -1505,6 +1513,10 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     const uint32_t nb = (n_rays + group - 1) / group;
     st = ensure_block_u32(ctx, 2 * (size_t)nb);
     if (st != TN_OK) return st;
+    // per-ray step positions for the emit pass
+    const uint32_t slot_cap = slot_capacity(n_rays, march->max_steps);
+    st = ensure_slots(ctx, (size_t)n_rays * slot_cap);
+    if (st != TN_OK) return st;
     // coarse mip of the bitfield, the per-level boxes of occupied blocks (ctx->box) and the bit-planes:
     // ctx->mip = [mip (R^3/64 B) | planes (n_levels x R^3/8 B, 256-byte aligned)]
     const int res = grid->resolution;
@@ -1522,10 +1534,6 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
         st = check_launch("tn_march_count(mip)");
         if (st != TN_OK) return st;
     }
-    // per-ray step positions for the emit pass
-    const uint32_t slot_cap = slot_capacity(n_rays, march->max_steps);
-    st = ensure_slots(ctx, (size_t)n_rays * slot_cap);
-    if (st != TN_OK) return st;
     ctx->slot_cap = slot_cap;
     ctx->slot_rays = n_rays;
     size_t smem = (use_mip ? mip_bytes : (size_t)12 * res) + (size_t)COUNT_RING * group;
@@ -1547,7 +1555,10 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
         default: st = TN_COUNT(COUNT_BYTES, COUNT_DEPTH_SHARED);
     }
 #undef TN_COUNT
-    if (st != TN_OK) return st;
+    if (st != TN_OK) {
+        if (use_mip) empty_box(ctx, stream);  // filled by the build, and no count to empty it
+        return st;
+    }
     ctx->count_group_used = group;
     return TN_OK;
 }
