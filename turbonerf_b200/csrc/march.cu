@@ -348,14 +348,16 @@ struct CountGrid {
 };
 
 // Forms of the count loop, picked on the host from the grid and the box (make_count_grid):
-//  BYTES    no coarse mip (R < 16 or R > 128): the bitfield byte of every step is read;
+//  BYTES    no coarse mip (R < 16 or R > 128) and a bitfield that starts at any byte: the byte of every
+//           step is read, without running ahead;
+//  WORDS    no coarse mip, the bitfield at a multiple of 4: the word of the step's byte is read;
 //  MIP      coarse mip and bit-planes, any geometry;
 //  BOUNDED  and the box lies inside the coarsest level, so that every scaled cell coordinate is in
 //           [0, R] (a size times its rounded reciprocal rounds to at most 1) and floor is one
 //           round-down addition: no conversion instructions;
 //  POW2     and the level sizes are powers of two, so that x times the level's scale is exact and
 //           the scaled coordinate is one fused multiply-add.
-enum CountMode : int { COUNT_BYTES = 0, COUNT_MIP = 1, COUNT_BOUNDED = 2, COUNT_POW2 = 3 };
+enum CountMode : int { COUNT_BYTES = 0, COUNT_WORDS = 1, COUNT_MIP = 2, COUNT_BOUNDED = 3, COUNT_POW2 = 4 };
 
 // get_grid_level_at (occupancy-grid.cuh:232-248): the finest level whose extent holds the point
 // (max |coordinate| m < half extent) and whose cell is larger than dt, else the coarsest. Each
@@ -496,6 +498,9 @@ __device__ __forceinline__ uint32_t read_word(uint32_t src) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(src));
     return v;
 }
+__device__ __forceinline__ void write_word(uint32_t dst, uint32_t v) {
+    asm volatile("st.shared.u32 [%0], %1;" ::"r"(dst), "r"(v));
+}
 __device__ __forceinline__ void store_if(bool on, float* p, float v) {
     asm volatile("{ .reg .pred p; setp.ne.u32 p, %0, 0; @p st.global.f32 [%1], %2; }" ::"r"((uint32_t)on), "l"(p), "f"(v));
 }
@@ -507,7 +512,7 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
                                    uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
                                    const uint32_t* __restrict__ spread, uint32_t ring, float* __restrict__ slots,
                                    uint32_t slot_cap) {
-    constexpr bool MIP = MODE != COUNT_BYTES;
+    constexpr bool MIP = MODE >= COUNT_MIP;
     constexpr bool FAST = MODE >= COUNT_BOUNDED;
     const float hx = __fmul_rn(0.5f, copysignf(1.0f, r.dx));
     const float hy = __fmul_rn(0.5f, copysignf(1.0f, r.dy));
@@ -583,7 +588,10 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
                 bit[j] = (cz << 4 & ~15u) | (((cy << 2 & 12u) | (cx & ~12u)) & 15u);  // taken modulo 32
             } else {
                 const uint32_t idx = spread[cx] | spread[res + cy] | spread[2 * res + cz];
-                fetch_word(ring + j * 4, reinterpret_cast<const uint32_t*>(cg.bits) + (idx >> 2), 4u);
+                if (MODE == COUNT_WORDS)
+                    fetch_word(ring + j * 4, reinterpret_cast<const uint32_t*>(cg.bits) + (idx >> 2), 4u);
+                else
+                    write_word(ring + j * 4, (uint32_t)__ldg(cg.bits + idx) << ((idx & 3u) * 8u));
                 bit[j] = 31u - (idx & 3u) * 8u - (uint32_t)k;
             }
             fetch_commit();
@@ -636,8 +644,8 @@ __device__ __forceinline__ uint32_t count_ray(const MarchArgs& a, const CountGri
         if (safe)
             return count_ray_loop<MODE, D, false>(a, cg, r, t_lim, max_steps, flags, mip, spread, ring, slots, slot_cap);
     }
-    return count_ray_loop<MODE == COUNT_BYTES ? COUNT_BYTES : COUNT_MIP, D, true>(a, cg, r, t_lim, max_steps, flags,
-                                                                                  mip, spread, ring, slots, slot_cap);
+    return count_ray_loop<MODE <= COUNT_MIP ? MODE : COUNT_MIP, D, true>(a, cg, r, t_lim, max_steps, flags, mip,
+                                                                         spread, ring, slots, slot_cap);
 }
 
 // World-space box that holds every occupied cell of every level: per level, the box of its
@@ -709,7 +717,7 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
                    uint32_t batch_size, uint32_t* batch_info, uint32_t* block_agg, uint32_t* block_prefix,
                    uint32_t* ticket, uint32_t* flags, const uint8_t* __restrict__ mip_g,
                    int* box_g, float* __restrict__ slots, uint32_t slot_cap) {
-    constexpr bool MIP = MODE != COUNT_BYTES;
+    constexpr bool MIP = MODE >= COUNT_MIP;
     extern __shared__ __align__(16) uint8_t smem[];
     uint32_t* spread = reinterpret_cast<uint32_t*>(smem);
     uint8_t* mip = smem;
@@ -1119,6 +1127,9 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
                         case COUNT_MIP:
                             cnt = count_ray<COUNT_MIP, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                             break;
+                        case COUNT_WORDS:
+                            cnt = count_ray<COUNT_WORDS, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            break;
                         default:
                             cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
                     }
@@ -1369,7 +1380,7 @@ static int make_count_grid(const MarchArgs& a, CountGrid& cg) {
                        std::isnormal(scale0 * dn),
                    TN_E_INVALID, "march: base_size %g out of range for %d levels", g.base, g.n_levels);
     }
-    cg.mode = COUNT_BYTES;
+    cg.mode = ((uintptr_t)g.bits & 3u) == 0 ? COUNT_WORDS : COUNT_BYTES;
     if (g.res >= MIP_MIN_RES && g.res <= MIP_MAX_RES) {
         const tn_bbox& b = a.bbox;
         float reach = 0.0f;
@@ -1411,7 +1422,7 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
         chunk += (sc.n_rays + chunk_rays - 1) >> A.chunk_shift;
         const int res = sc.grid.resolution;
         max_res = std::max<uint32_t>(max_res, (uint32_t)res);
-        sp.use_mip = sp.cg.mode != COUNT_BYTES;
+        sp.use_mip = sp.cg.mode >= COUNT_MIP;
         sp.cshift = sp.cg.res_shift - 2;
         if (sp.use_mip) {
             TN_REQUIRE(((uintptr_t)sc.bitfield & 15u) == 0, TN_E_INVALID, "scene %u: bitfield must be 16-byte aligned", s);
@@ -1520,7 +1531,7 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     // coarse mip of the bitfield, the per-level boxes of occupied blocks (ctx->box) and the bit-planes:
     // ctx->mip = [mip (R^3/64 B) | planes (n_levels x R^3/8 B, 256-byte aligned)]
     const int res = grid->resolution;
-    const bool use_mip = cg.mode != COUNT_BYTES;
+    const bool use_mip = cg.mode >= COUNT_MIP;
     const uint32_t mip_bytes = use_mip ? (uint32_t)(res / 4) * (res / 4) * (res / 4) : 0u;
     const size_t planes_off = ((size_t)mip_bytes + 255) & ~(size_t)255;
     if (use_mip) {
@@ -1552,6 +1563,7 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
             st = shared ? TN_COUNT(COUNT_BOUNDED, COUNT_DEPTH_SHARED) : TN_COUNT(COUNT_BOUNDED, COUNT_DEPTH);
             break;
         case COUNT_MIP: st = TN_COUNT(COUNT_MIP, COUNT_DEPTH_SHARED); break;
+        case COUNT_WORDS: st = TN_COUNT(COUNT_WORDS, COUNT_DEPTH_SHARED); break;
         default: st = TN_COUNT(COUNT_BYTES, COUNT_DEPTH_SHARED);
     }
 #undef TN_COUNT
