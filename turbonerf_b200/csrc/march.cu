@@ -337,6 +337,7 @@ struct CountGrid {
     int scale0_bits;             // bit pattern of R / level-0 size
     uint32_t res_m1;             // R - 1
     int res_shift;               // log2 R
+    uint32_t spread_pitch;       // entries of each Morton spread table (R; several scenes share the largest's)
     int level_max;               // number of levels - 1
     float res_below;             // the float below R
     int mode;                    // CountMode
@@ -517,7 +518,7 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
     const float hx = __fmul_rn(0.5f, copysignf(1.0f, r.dx));
     const float hy = __fmul_rn(0.5f, copysignf(1.0f, r.dy));
     const float hz = __fmul_rn(0.5f, copysignf(1.0f, r.dz));
-    const uint32_t C = 1u << (cg.res_shift - 2), C3 = C * C * C, res = 1u << cg.res_shift;
+    const uint32_t C = 1u << (cg.res_shift - 2), C3 = C * C * C;
     const uint32_t max_iters = a.max_iters;
     // the loop's constants in registers: read from the parameters they would be loaded again each trip
     const float cone = in_reg(a.cone), dt_min = in_reg(a.dt_min), dt_max = in_reg(a.dt_max);
@@ -587,7 +588,7 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
                            ((uint32_t)mip[blk] >> k << 2) & 4u);
                 bit[j] = (cz << 4 & ~15u) | (((cy << 2 & 12u) | (cx & ~12u)) & 15u);  // taken modulo 32
             } else {
-                const uint32_t idx = spread[cx] | spread[res + cy] | spread[2 * res + cz];
+                const uint32_t idx = spread[cx] | spread[cg.spread_pitch + cy] | spread[2 * cg.spread_pitch + cz];
                 if (MODE == COUNT_WORDS)
                     fetch_word(ring + j * 4, reinterpret_cast<const uint32_t*>(cg.bits) + (idx >> 2), 4u);
                 else
@@ -1368,6 +1369,7 @@ static int make_count_grid(const MarchArgs& a, CountGrid& cg) {
     cg.cell0_below = cg.cell0_bits - (1 << 23);
     cg.res_shift = 0;
     while ((1 << cg.res_shift) < g.res) ++cg.res_shift;
+    cg.spread_pitch = (uint32_t)g.res;
     cg.level_max = g.n_levels - 1;
     cg.res_below = std::nextafter(g.res_f, 0.0f);
     cg.bits = g.bits;
@@ -1441,6 +1443,7 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
     A.total_chunks = chunk;
     A.total_rays = prev_end;
     A.spread_res = max_res;
+    for (uint32_t s = 0; s < n_scenes; ++s) A.sp[s].cg.spread_pitch = max_res;
     if (build_scratch && scratch) {
         const int st = ensure_mip(ctx, scratch);
         if (st != TN_OK) return st;
