@@ -784,12 +784,17 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
 constexpr int EXPAND_U = 4;
 
 // The march of ray r from its occupied step at t on: writes the positions of the next n >= 1 occupied
-// steps (which the count pass found) and returns the last one.
+// steps (which the count pass found) and returns the last one. A march over inputs that have changed since
+// the count may not find them: once it steps through empty cells outside the cube around the box, or past
+// the iteration limit, it stands still, as the reference's emit loop does past the box, and what is left
+// of the n positions is where it stands. Only empty steps are checked; occupied ones end by themselves.
 __device__ float replay_steps(const MarchArgs& a, const RayMarch& r, float t, uint32_t n, float* out) {
+    const float reach = fmaxf(fmaxf(fmaxf(fabsf(a.bbox.min_x), fabsf(a.bbox.max_x)),
+                                    fmaxf(fabsf(a.bbox.min_y), fabsf(a.bbox.max_y))),
+                              fmaxf(fabsf(a.bbox.min_z), fabsf(a.bbox.max_z)));
     float last = t;
     t = __fadd_rn(t, get_dt(t, a.cone, a.dt_min, a.dt_max));
-    // the count pass bounded this loop; the limit only protects against inputs that changed since
-    for (uint32_t taken = 0, iters = 0; taken < n && iters < a.max_iters; ++iters) {
+    for (uint32_t taken = 0, iters = 0; taken < n; ++iters) {
         float x, y, z;
         ray_point(r, t, x, y, z);
         const float dt = get_dt(t, a.cone, a.dt_min, a.dt_max);
@@ -797,6 +802,8 @@ __device__ float replay_steps(const MarchArgs& a, const RayMarch& r, float t, ui
         if (occupied_at(a.g, k, x, y, z)) {
             out[taken++] = last = t;
             t = __fadd_rn(t, dt);
+        } else if (!(fmaxf(fabsf(x), fmaxf(fabsf(y), fabsf(z))) <= reach) || iters >= a.max_iters) {
+            out[taken++] = t;
         } else {
             t = __fadd_rn(t, dt_to_next_voxel(a.g, x, y, z, r.dx, r.dy, r.dz, r.idx, r.idy, r.idz, a.dt_min, k));
         }
