@@ -390,13 +390,17 @@ __device__ __forceinline__ uint32_t live_rays(uint32_t n_rays, const uint32_t* n
     return n_dev ? min(*n_dev, n_rays) : n_rays;
 }
 
-// Two lower bounds at once over ascending offsets: the first i < n with off[i] >= va (lanes
-// 0-15) and >= vb (lanes 16-31), n where there is none. Each half probes 16 positions a round and
+// Samples that a ray counts for in the balanced split, beside its own (balanced_rays).
+constexpr uint32_t RAY_COST = 2;
+
+// Two lower bounds at once over ascending offsets: the first i < n with off[i] + RAY_COST i >= va
+// (lanes 0-15) and >= vb (lanes 16-31), n where there is none. Each half probes 16 positions a round and
 // keeps the sub-range where the offsets cross its value; every lane of the warp runs every round.
-__device__ uint2 warp_lower_bounds(const uint32_t* __restrict__ off, uint32_t n, uint32_t va, uint32_t vb, int lane) {
+__device__ uint2 warp_lower_bounds(const uint32_t* __restrict__ off, uint32_t n, uint64_t va, uint64_t vb, int lane) {
     const int half = lane >> 4, j = lane & 15;
-    const uint32_t v = half ? vb : va;
-    uint32_t lo = 0, hi = n;  // the answer lies in [lo, hi]; hi == n or off[hi] >= v
+    const uint64_t v = half ? vb : va;
+    auto reaches = [&](uint32_t i) { return off[i] + (uint64_t)RAY_COST * i >= v; };
+    uint32_t lo = 0, hi = n;  // the answer lies in [lo, hi]; hi == n or hi reaches v
     for (;;) {
         const bool active = hi - lo > 16u;
         if (__ballot_sync(FULL_MASK, active) == 0u) break;
@@ -404,7 +408,7 @@ __device__ uint2 warp_lower_bounds(const uint32_t* __restrict__ off, uint32_t n,
         bool pred = false;
         if (active) {
             step = (hi - lo + 15u) / 16u;
-            pred = off[min(lo + (uint32_t)(j + 1) * step, hi) - 1u] >= v;
+            pred = reaches(min(lo + (uint32_t)(j + 1) * step, hi) - 1u);
         }
         const unsigned m = (__ballot_sync(FULL_MASK, pred) >> (16 * half)) & 0xFFFFu;
         if (active) {
@@ -418,20 +422,25 @@ __device__ uint2 warp_lower_bounds(const uint32_t* __restrict__ off, uint32_t n,
             }
         }
     }
-    const bool pred = lo + (uint32_t)j < hi && off[lo + (uint32_t)j] >= v;
+    const bool pred = lo + (uint32_t)j < hi && reaches(lo + (uint32_t)j);
     const unsigned m = (__ballot_sync(FULL_MASK, pred) >> (16 * half)) & 0xFFFFu;
     const uint32_t ans = m ? lo + (uint32_t)(__ffs(m) - 1) : hi;
     return make_uint2(__shfl_sync(FULL_MASK, ans, 0), __shfl_sync(FULL_MASK, ans, 16));
 }
 
-// The rays of warp w of W under a sample-balanced split: those whose first sample lies in
-// [w S / W, (w + 1) S / W), S the batch's samples (offsets ascending); the last warp also takes
-// the rays without samples at the end.
+// The rays of warp w of W under a balanced split: those whose first sample, every ray counting for
+// RAY_COST samples more, lies in [w S / W, (w + 1) S / W), S the batch's samples and RAY_COST a ray
+// (offsets ascending). Without the rays' own cost a run of rays without samples, an image's
+// background, all went to one warp: 2^20 samples in 2^17 rays with as many empty ones between them, distortion
+// loss and gradient 12.2 ms, compositor forward and gradient 0.93 and 1.01; with a cost of 1, 2, 4, 8
+// samples 56, 40, 37, 37 us, 18.6, 20.3, 21.4, 21.9 and 16.5, 16.5, 16.5, 15.0; half of 1.6 million rays empty
+// at the end (mean of the others 5) 117, 127, 139, 154, 70, 75, 83, 88 and 57, 62, 66, 72. Batches without such
+// runs are as fast with 2 as without, or faster (5e5 samples, mean 6: 23.6 -> 20.6 and 12.4 -> 10.4).
 __device__ __forceinline__ uint2 balanced_rays(const uint32_t* __restrict__ counts,
                                                const uint32_t* __restrict__ offsets, uint32_t n_live, uint32_t w,
                                                uint32_t W, int lane) {
-    const uint32_t total = offsets[n_live - 1] + counts[n_live - 1];
-    const uint32_t va = (uint32_t)((uint64_t)total * w / W), vb = (uint32_t)((uint64_t)total * (w + 1) / W);
+    const uint64_t total = (uint64_t)offsets[n_live - 1] + counts[n_live - 1] + (uint64_t)RAY_COST * n_live;
+    const uint64_t va = total * w / W, vb = total * (w + 1) / W;
     uint2 r = warp_lower_bounds(offsets, n_live, va, vb, lane);
     if (w == 0) r.x = 0;
     if (w + 1 == W) r.y = n_live;
