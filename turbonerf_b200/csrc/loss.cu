@@ -1093,8 +1093,8 @@ composite_bwd_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, ui
 // ---- distortion loss over sample tiles ------------------------------------------------------
 // The distortion loss forward and backward (mipNeRF360_distortion_loss_forward_kernel /
 // _backward_kernel, training-kernels-fused.cuh:13-224, with the sums A, B above) in the tile
-// form of the compositor: a warp takes the rays that start in its share of the samples
-// (balanced_rays), in groups of at most `group`, and walks a group's samples in tiles of
+// form of the compositor: a warp takes one ray, or where there are more rays than warps those that start in
+// its share of the samples (balanced_rays), in groups of at most `group`, and walks a group's samples in tiles of
 // 32 * K, lane l owning K consecutive samples. Forward, tiles in increasing order: per sample the
 // optical depth before it, the weight w = T (1 - e^-x), the weight sum before it W_<, the
 // increment dm of m and A = sum dm W_<, each a segmented scan of the lane aggregates with a
@@ -1110,10 +1110,11 @@ composite_bwd_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, ui
 // Bound by instruction issue (dependent scans, 24 warps an SM), not by its 12 or 16 bytes a sample
 // (8 and 11 us at 2^22 samples). The shares are of samples: with the same number of rays a warp,
 // one wave ended with the warp whose rays happened to be long (geometric lengths, 19 rays a warp:
-// 1.5 to 1.8 times the mean). Loss launch and gradient launch, mean 64 samples a ray, 2^22 samples:
-// 46.2 and 108.8 us before, 38.0 and 69.9 now; 5e5 samples, mean 128: 22.8 and 57.7, 20.2 and 41.2;
-// 4e6, mean 5: 66.9 and 123.6, 57.2 and 84.0; 6e4, mean 20: 9.0 and 16.0, 6.6 and 11.6. Loss of 5e5
-// samples, mean 6: 10.7, 11.7 now (the search for the shares), its gradient 21.4, 16.5.
+// 1.5 to 1.8 times the mean). Loss launch, gradient launch and both in one, the same number of rays a warp
+// against shares: 2^22 samples, mean 64: 43.2, 90.3 and 93.3 us, 37.0, 64.7 and 74.1; 5e5, mean 128: 20.6,
+// 39.1 and 41.1, 22.7, 35.0 and 41.1; 4e6, mean 5: 55.4, 96.5 and 104, 52.6, 74.0 and 101; 2^18, mean 48: 12.4,
+// 18.6 and 22.6, 14.4, 16.5 and 22.6; 5e5, mean 6: 12.4, 17.0 and 20.3, 13.5, 14.5 and 20.6. A loss alone at about
+// a tile a warp is the one that loses, 2 us, the search for the shares.
 
 struct DistTile {
     float sig[ST_K], dtn[ST_K], w[ST_K], tn[ST_K], dm[ST_K], a[ST_K];
@@ -1252,8 +1253,9 @@ distortion_tiles_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint3
     __shared__ float t_k[LOSS_WARPS][WARP], t_gs[LOSS_WARPS][WARP];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const uint32_t n_live = live_rays(n_rays, n_dev);
-    uint2 rr = make_uint2(0u, 0u);
-    if (n_live) rr = balanced_rays(counts, offsets, n_live, blockIdx.x * LOSS_WARPS + wid, gridDim.x * LOSS_WARPS, lane);
+    const uint32_t w = blockIdx.x * LOSS_WARPS + wid, W = gridDim.x * LOSS_WARPS;
+    uint2 rr = make_uint2(min(w, n_live), min(w + 1, n_live));  // a ray a warp, while the warps suffice
+    if (n_rays > W && n_live) rr = balanced_rays(counts, offsets, n_live, w, W, lane);
     float acc[1] = {0.0f};
     for (uint32_t r0 = rr.x; r0 < rr.y; r0 += group) {  // whole warps; every thread reaches the block sum below
         const int nr = (int)min(group, rr.y - r0);
@@ -2622,8 +2624,11 @@ static int launch_train_losses(tn_ctx* ctx, cudaStream_t stream, const tn_ray_ba
 // Blocks of the distortion tiles: by the batch's mean samples per ray (sample_stride / n_rays, an
 // upper bound) about one tile (32 * ST_K samples) a warp while that leaves warps per SM idle, up
 // to 4 when it does not (the setup of a warp's range and its partly filled first and last tiles
-// are then paid once per 4 tiles), and at most one wave of resident warps. `group`: rays of at
-// most 32 tiles on average, half of those whose carries a warp keeps.
+// are then paid once per 4 tiles), and at most one wave of resident warps. A batch of no more rays than
+// that wave has warps takes a warp a ray and needs no shares: they gave some warps two of the long rays and
+// others none (700 rays of 1500 samples, loss and gradient: 371 us by shares, 313 a ray a warp), and the
+// search for them is a good part of a short launch (3000 rays of 20: 14.5, 12.4; 655 of 400: 82, 76).
+// `group`: rays of at most 32 tiles on average, half of those whose carries a warp keeps.
 static int distortion_grid(const tn_ray_batch* b, const void* kernel, uint32_t& group) {
     const double mean = b->n_rays ? std::max(1.0, (double)b->sample_stride / (double)b->n_rays) : 1.0;
     const double per_tile = (double)(WARP * ST_K);
@@ -2632,7 +2637,7 @@ static int distortion_grid(const tn_ray_batch* b, const void* kernel, uint32_t& 
     const uint32_t rpw = (uint32_t)std::min(32.0, std::max(1.0, std::floor(tiles * per_tile / mean)));
     group = (uint32_t)std::min(32.0, std::max(1.0, std::floor(SAVED_TILES / 2 * per_tile / mean)));
     const uint32_t wave = (uint32_t)num_sms() * (uint32_t)blocks_per_sm(kernel, LOSS_THREADS);
-    const uint32_t warps = (b->n_rays + rpw - 1) / rpw;
+    const uint32_t warps = b->n_rays <= wave * LOSS_WARPS ? b->n_rays : (b->n_rays + rpw - 1) / rpw;
     return (int)std::min(wave, (warps + LOSS_WARPS - 1) / LOSS_WARPS);
 }
 
