@@ -229,45 +229,88 @@ hg_backward_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev,
 }
 
 // Lists every entry a live sample touches once (the thread whose atomic or sets the entry's bit appends
-// l T + idx), one thread per (sample, level). A bit already set is seen with a plain read and skips
-// its atomic; the lanes of a warp that share an entry send one of them; the warp's new entries
-// take one counter atomic for the warp.
+// l T + idx), one thread per (sample, level); with ADD it adds the sample's gradients too, one launch for
+// a short batch. A cell shared with the sample before, as along a ray, is that one's to list; bits already
+// set are seen with a plain read and skip their atomic; the two corners of an x edge have theirs in one word
+// for 31 of 32 x, read and set as one; a block's new entries take one counter atomic.
+// Bound by the L2's atomics with a result (about 17 G a second; one a new entry is what the edges halve) and
+// by random reads. The backward with its list, 2^18 samples of 16 levels along rays and uniform: 310 and
+// 485 us; 467 and 590 where one kernel added and listed a sample a thread, 416 and 609 with this kernel
+// one atomic a corner, lanes compared entry by entry and one counter atomic a warp. Listing inside
+// the runs of hg_backward_kernel, edges together: 375 and 424, but 8000 samples 30 and 28 where this takes 22 and 25.
+template <bool ADD>
 __global__ void __launch_bounds__(HG_THREADS)
-hg_touch_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t pstride,
-                const float* __restrict__ pos, uint32_t* __restrict__ bits, uint32_t* __restrict__ list,
-                uint32_t* __restrict__ count) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+hg_touch_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev, uint32_t pstride, uint32_t stride,
+                const float* __restrict__ pos, const float* __restrict__ dfeat, float2* __restrict__ grads, bool pairs,
+                uint32_t* __restrict__ bits, uint32_t* __restrict__ list, uint32_t* __restrict__ count) {
+    __shared__ uint32_t warp_n[HG_THREADS / WARP];
+    __shared__ uint32_t block_at;
+    const uint32_t nl = live_count(n, n_dev);
+    if (blockIdx.x * HG_THREADS >= nl) return;  // whole blocks
+    const uint32_t s = blockIdx.x * HG_THREADS + threadIdx.x, at_s = min(s, nl - 1u);
     const int l = blockIdx.y;
-    const int lane = threadIdx.x & 31;
-    const bool live = s < live_count(n, n_dev);
-    const unsigned active = __ballot_sync(FULL_MASK, live);  // the warp's lanes that continue together
-    if (!live) return;
-    const HashCell c = hg_locate(H, l, pos[s], pos[s + pstride], pos[s + 2 * (size_t)pstride]);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const HashCell c = hg_locate(H, l, pos[at_s], pos[at_s + pstride], pos[at_s + 2 * (size_t)pstride]);
+    HashCell before = c;
+    before.x = __shfl_up_sync(FULL_MASK, c.x, 1);
+    before.y = __shfl_up_sync(FULL_MASK, c.y, 1);
+    before.z = __shfl_up_sync(FULL_MASK, c.z, 1);
+    const bool head = s < nl && (lane == 0 || !hg_same(before, c));
     const uint32_t base = (uint32_t)l << H.log2_t;
+    // the two corners of an x edge have their bits in one word for 31 of 32 x
     uint32_t e[8], word[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
+    for (int k = 0; k < 8; k += 2) {
         e[k] = base + hg_corner(H, l, c, k);
-        word[k] = lane == __ffs(__match_any_sync(active, e[k])) - 1 ? bits[e[k] >> 5] : ~0u;
+        e[k + 1] = base + hg_corner(H, l, c, k + 1);
+        word[k] = head ? bits[e[k] >> 5] : ~0u;
+        word[k + 1] = !head ? ~0u : (e[k] ^ e[k + 1]) < 32u ? word[k] : bits[e[k + 1] >> 5];
+    }
+    if (ADD && s < nl) {  // beside the words on their way
+        const float g0 = dfeat[(size_t)(HG_F * l) * stride + s], g1 = dfeat[(size_t)(HG_F * l + 1) * stride + s];
+        float w[8];
+        hg_weights(c, w);
+        float2 g[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) g[k] = make_float2(__fmul_rn(w[k], g0), __fmul_rn(w[k], g1));
+        hg_flush(H, l, c, g, grads + base, pairs);
     }
     bool fresh[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const uint32_t bit = 1u << (e[k] & 31u);
-        fresh[k] = !(word[k] & bit) && !(atomicOr(bits + (e[k] >> 5), bit) & bit);
+    for (int k = 0; k < 8; k += 2) {
+        const bool together = (e[k] ^ e[k + 1]) < 32u;
+        uint32_t b0 = ~word[k] & (1u << (e[k] & 31u)), b1 = ~word[k + 1] & (1u << (e[k + 1] & 31u));
+        const uint32_t set = together ? b0 | b1 : b0;
+        if (set) {
+            const uint32_t old = atomicOr(bits + (e[k] >> 5), set);
+            b0 &= ~old;
+            if (together) b1 &= ~old;
+        }
+        if (!together && b1) b1 &= ~atomicOr(bits + (e[k + 1] >> 5), b1);
+        fresh[k] = b0 != 0u;
+        fresh[k + 1] = b1 != 0u;
     }
     unsigned news[8];
     uint32_t total = 0;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
-        news[k] = __ballot_sync(active, fresh[k]);
+        news[k] = __ballot_sync(FULL_MASK, fresh[k]);
         total += (uint32_t)__popc(news[k]);
     }
-    if (total == 0) return;
-    const int first = __ffs(active) - 1;
-    uint32_t at = 0;
-    if (lane == first) at = atomicAdd(count, total);
-    at = __shfl_sync(active, at, first);
+    if (lane == 0) warp_n[wid] = total;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t sum = 0;
+#pragma unroll
+        for (int w = 0; w < HG_THREADS / WARP; ++w) {
+            const uint32_t v = warp_n[w];
+            warp_n[w] = sum;
+            sum += v;
+        }
+        block_at = sum ? atomicAdd(count, sum) : 0u;
+    }
+    __syncthreads();
+    uint32_t at = block_at + warp_n[wid];
     const unsigned below = (1u << lane) - 1u;
 #pragma unroll
     for (int k = 0; k < 8; ++k) {
@@ -507,6 +550,16 @@ int hashgrid_backward(cudaStream_t stream, const tn_hashgrid_desc* desc, uint32_
 #define TN_HG_BACKWARD(RUN, VEC)                                                                           \
     hg_backward_kernel<RUN, VEC><<<hg_grid(n, H.n_levels, RUN), HG_THREADS, 0, stream>>>(H, n, n_dev, pstride, \
                                                                                        stride, pos, dL_dfeatures, G, pairs)
+#define TN_HG_TOUCH(ADD)                                                                                            \
+    hg_touch_kernel<ADD><<<hg_grid(n, H.n_levels, 1), HG_THREADS, 0, stream>>>(                                      \
+        H, n, n_dev, pstride, stride, pos, dL_dfeatures, G, pairs, touched_bits, touched_list, touched_count)
+    // With a list, up to 2^17 (sample, level) pairs one launch adds and lists (1000 samples of 16 levels 15.4
+    // us against 20.5 in two; 8000 uniform 25.3 against 27.7); past it the runs are worth their own (30,000 along
+    // rays 50.2 against 46.1, 65,536 97 against 83).
+    if (touched_bits && (uint64_t)n * H.n_levels <= (1u << 17)) {
+        TN_HG_TOUCH(true);
+        return check_launch("tn_hashgrid_backward");
+    }
     // Eight samples a thread from 2^20 (sample, level) pairs on (2^18 samples, 16 levels: 85 us against
     // 89 with four), four below, where the GPU wants more threads (8000 samples: 5.9 against 9.1 us;
     // even at 64,000).
@@ -518,9 +571,8 @@ int hashgrid_backward(cudaStream_t stream, const tn_hashgrid_desc* desc, uint32_
         else TN_HG_BACKWARD(4, false);
     }
 #undef TN_HG_BACKWARD
-    if (touched_bits)
-        hg_touch_kernel<<<hg_grid(n, H.n_levels, 1), HG_THREADS, 0, stream>>>(H, n, n_dev, pstride, pos, touched_bits,
-                                                                            touched_list, touched_count);
+    if (touched_bits) TN_HG_TOUCH(false);
+#undef TN_HG_TOUCH
     return check_launch("tn_hashgrid_backward");
 }
 
