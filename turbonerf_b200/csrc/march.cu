@@ -337,7 +337,6 @@ struct CountGrid {
     int scale0_bits;             // bit pattern of R / level-0 size
     uint32_t res_m1;             // R - 1
     int res_shift;               // log2 R
-    uint32_t spread_pitch;       // entries of each Morton spread table (R; several scenes share the largest's)
     int level_max;               // number of levels - 1
     float res_below;             // the float below R
     int mode;                    // CountMode
@@ -511,8 +510,8 @@ __device__ __forceinline__ void store_if(bool on, float* p, float v) {
 template <int MODE, int D, bool GUARD>
 __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, const RayMarch& r, float t_lim,
                                    uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
-                                   const uint32_t* __restrict__ spread, uint32_t ring, float* __restrict__ slots,
-                                   uint32_t slot_cap) {
+                                   const uint32_t* __restrict__ spread, uint32_t spread_pitch, uint32_t ring,
+                                   float* __restrict__ slots, uint32_t slot_cap) {
     constexpr bool MIP = MODE >= COUNT_MIP;
     constexpr bool FAST = MODE >= COUNT_BOUNDED;
     const float hx = __fmul_rn(0.5f, copysignf(1.0f, r.dx));
@@ -588,7 +587,7 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
                            ((uint32_t)mip[blk] >> k << 2) & 4u);
                 bit[j] = (cz << 4 & ~15u) | (((cy << 2 & 12u) | (cx & ~12u)) & 15u);  // taken modulo 32
             } else {
-                const uint32_t idx = spread[cx] | spread[cg.spread_pitch + cy] | spread[2 * cg.spread_pitch + cz];
+                const uint32_t idx = spread[cx] | spread[spread_pitch + cy] | spread[2 * spread_pitch + cz];
                 if (MODE == COUNT_WORDS)
                     fetch_word(ring + j * 4, reinterpret_cast<const uint32_t*>(cg.bits) + (idx >> 2), 4u);
                 else
@@ -629,8 +628,8 @@ __device__ uint32_t count_ray_loop(const MarchArgs& a, const CountGrid& cg, cons
 template <int MODE, int D>
 __device__ __forceinline__ uint32_t count_ray(const MarchArgs& a, const CountGrid& cg, const RayMarch& r, float t_lim,
                                               uint32_t max_steps, uint32_t* flags, const uint8_t* __restrict__ mip,
-                                              const uint32_t* __restrict__ spread, uint32_t ring,
-                                              float* __restrict__ slots, uint32_t slot_cap) {
+                                              const uint32_t* __restrict__ spread, uint32_t spread_pitch,
+                                              uint32_t ring, float* __restrict__ slots, uint32_t slot_cap) {
     if (!(r.t <= t_lim)) return 0;  // no step (a NaN limit included)
     float x, y, z;
     ray_point(r, r.t, x, y, z);
@@ -643,10 +642,11 @@ __device__ __forceinline__ uint32_t count_ray(const MarchArgs& a, const CountGri
         const bool safe = a.dt_min >= far * 4.8e-7f && fminf(fminf(fabsf(r.idx), fabsf(r.idy)), fabsf(r.idz)) < 1e30f &&
                           (t_lim - r.t) < 0.8f * a.dt_min * (float)(a.max_iters >> 1);
         if (safe)
-            return count_ray_loop<MODE, D, false>(a, cg, r, t_lim, max_steps, flags, mip, spread, ring, slots, slot_cap);
+            return count_ray_loop<MODE, D, false>(a, cg, r, t_lim, max_steps, flags, mip, spread, spread_pitch, ring,
+                                                  slots, slot_cap);
     }
     return count_ray_loop<MODE <= COUNT_MIP ? MODE : COUNT_MIP, D, true>(a, cg, r, t_lim, max_steps, flags, mip,
-                                                                         spread, ring, slots, slot_cap);
+                                                                         spread, spread_pitch, ring, slots, slot_cap);
 }
 
 // World-space box that holds every occupied cell of every level: per level, the box of its
@@ -763,8 +763,9 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
             const float below = nextafterf(t_max, -INFINITY);
             const float t_lim = t_stop < below ? t_stop : below;  // a NaN t_max stays NaN
             if (meets)
-                cnt = count_ray<MODE, D>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip, spread, ring,
-                                      slots ? slots + (size_t)i * slot_cap : nullptr, slots ? slot_cap : 0u);
+                cnt = count_ray<MODE, D>(a, cg, r, t_lim, a.max_steps ? a.max_steps : 0xffffffffu, flags, mip, spread,
+                                      1u << cg.res_shift, ring, slots ? slots + (size_t)i * slot_cap : nullptr,
+                                      slots ? slot_cap : 0u);
             if (cnt == 0) alive[i] = 0;
         }
         counts[i] = cnt;
@@ -777,8 +778,12 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
                                      flags);
     if (threadIdx.x == 0) *ticket = 0u;
     // every block read the box before it took its ticket: the next call's build starts from an empty one
-    if (MIP)
-        for (int k = threadIdx.x; k < BOX_INTS; k += blockDim.x) box_g[k] = k < BOX_INTS / 2 ? BOX_EMPTY_LO : 0;
+    // (written as a loop over the box it cost the march loop 3%, by the code around it)
+    static_assert(BOX_INTS / 2 <= WARP, "one thread a bound, in the smallest block too");
+    if (MIP && threadIdx.x < BOX_INTS / 2) {
+        box_g[threadIdx.x] = BOX_EMPTY_LO;
+        box_g[BOX_INTS / 2 + threadIdx.x] = 0;
+    }
 }
 
 constexpr int EXPAND_U = 4;
@@ -1127,19 +1132,19 @@ multi_count_kernel(const __grid_constant__ MultiArgs A, uint32_t rs, const float
                 if (meets) {
                     switch (sp.cg.mode) {  // the same for the whole chunk
                         case COUNT_POW2:
-                            cnt = count_ray<COUNT_POW2, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_POW2, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, res, ring, sl, sc);
                             break;
                         case COUNT_BOUNDED:
-                            cnt = count_ray<COUNT_BOUNDED, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_BOUNDED, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, res, ring, sl, sc);
                             break;
                         case COUNT_MIP:
-                            cnt = count_ray<COUNT_MIP, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_MIP, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, res, ring, sl, sc);
                             break;
                         case COUNT_WORDS:
-                            cnt = count_ray<COUNT_WORDS, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_WORDS, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, res, ring, sl, sc);
                             break;
                         default:
-                            cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, ring, sl, sc);
+                            cnt = count_ray<COUNT_BYTES, COUNT_DEPTH_SHARED>(sp.a, sp.cg, r, t_lim, ms, flags, mip, spread, res, ring, sl, sc);
                     }
                 }
                 if (cnt == 0) alive[i] = 0;
@@ -1376,7 +1381,6 @@ static int make_count_grid(const MarchArgs& a, CountGrid& cg) {
     cg.cell0_below = cg.cell0_bits - (1 << 23);
     cg.res_shift = 0;
     while ((1 << cg.res_shift) < g.res) ++cg.res_shift;
-    cg.spread_pitch = (uint32_t)g.res;
     cg.level_max = g.n_levels - 1;
     cg.res_below = std::nextafter(g.res_f, 0.0f);
     cg.bits = g.bits;
@@ -1450,7 +1454,6 @@ static int make_multi_args(tn_ctx* ctx, uint32_t n_scenes, const tn_scene* scene
     A.total_chunks = chunk;
     A.total_rays = prev_end;
     A.spread_res = max_res;
-    for (uint32_t s = 0; s < n_scenes; ++s) A.sp[s].cg.spread_pitch = max_res;
     if (build_scratch && scratch) {
         const int st = ensure_mip(ctx, scratch);
         if (st != TN_OK) return st;
