@@ -465,13 +465,17 @@ __device__ __forceinline__ float box_exit_t(const tn_bbox& b, const RayMarch& r,
 // of 2.5e5 rays (persistent launch, many warps a scheduler) 1238 -> 730 us. Steps in flight (D) on
 // the first two: 3 84 and 158 us, 4 83 and 140, 5 78 and 134, 6 76 and 129, 8 78 and 118. Words kept in registers instead of shared memory cost 10% (the loads then
 // share the few scoreboards and wait for each other).
-// Steps in flight: 6 where the launch has the GPU to itself; 3 where it shares it with other work
-// (side_sms: blocks of 256 rays on a part of the SMs; the persistent launch), where other warps
-// hide the lookups and what a wrong guess wastes counts: a training step over a grid of random
-// cells (36% occupied) takes its count 449 us with 3 and 532 with 6, over smooth fields 160 and
-// 179. Alone, 6 wins or ties from 64 to 65,536 rays (2^16: 217 against 265 us).
+// Steps in flight: 6 where a scheduler has one warp at most, with the GPU to itself; 3 where other warps
+// hide the lookups (more rays than the schedulers take at a warp each, the persistent launch, or side_sms:
+// blocks of 256 rays on a part of the SMs) and what a wrong guess wastes counts: a training step over a
+// grid of random cells (36% occupied) takes its count 449 us with 3 and 532 with 6, over smooth fields 160
+// and 179. Alone, on either side of the line (18,944 rays), 6 and 3 steps: smooth field of 5 cascades
+// 2^14 rays 92 and 99 us, 20,000 rays 126 and 124, 2^16 241 and 238; one cascade at a fixed step 171 and 185,
+// 270 and 258, 2^16 1090 both; random cells, 30% occupied, 266 and 243, 443 and 306, 2^16 1256 and 956
+// (2^14 takes 6 for the smooth fields' sake).
 constexpr int COUNT_DEPTH = 6;
 constexpr int COUNT_DEPTH_SHARED = 3;
+constexpr uint32_t SCHEDULERS = 4;  // warp schedulers an SM
 constexpr int COUNT_RING = 4 * (COUNT_DEPTH | 1);  // bytes a thread of shared memory (an odd number of words: no bank conflicts)
 
 // Copies the word at p into shared memory asynchronously, or zero when `bytes` is 0 instead of 4.
@@ -777,12 +781,18 @@ march_count_kernel(MarchArgs a, CountGrid cg, uint32_t n_rays, const uint32_t* _
     scan_blocks_and_cut<COUNT_GROUP_MAX>(gridDim.x, n_live, counts, block_agg, block_prefix, batch_size, batch_info,
                                      flags);
     if (threadIdx.x == 0) *ticket = 0u;
-    // every block read the box before it took its ticket: the next call's build starts from an empty one
-    // (written as a loop over the box it cost the march loop 3%, by the code around it)
+    // Every block read the box before it took its ticket: the next call's build starts from an empty one.
+    // Which of the two shapes only matters to the march loop that the compiler makes beside it: with the
+    // other one 6 steps in flight take 3% longer (2^14 rays, random cells: 267 and 281 us), 3 steps 2 to 4%
+    // (2^16 rays, 5 cascades: 238 and 251).
     static_assert(BOX_INTS / 2 <= WARP, "one thread a bound, in the smallest block too");
-    if (MIP && threadIdx.x < BOX_INTS / 2) {
-        box_g[threadIdx.x] = BOX_EMPTY_LO;
-        box_g[BOX_INTS / 2 + threadIdx.x] = 0;
+    if (MIP && D == COUNT_DEPTH) {
+        if (threadIdx.x < BOX_INTS / 2) {
+            box_g[threadIdx.x] = BOX_EMPTY_LO;
+            box_g[BOX_INTS / 2 + threadIdx.x] = 0;
+        }
+    } else if (MIP) {
+        for (int k = threadIdx.x; k < BOX_INTS; k += blockDim.x) box_g[k] = k < BOX_INTS / 2 ? BOX_EMPTY_LO : 0;
     }
 }
 
@@ -1567,7 +1577,7 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
     launch_count<MODE, D>(nb, group, smem, stream, a, cg, n_rays, n_rays_dev, ray_stride, ori, dir, ray_t, ray_t_max, \
                           alive, n_steps, batch_size, batch_info, ctx->block_u32, ctx->block_u32 + nb,                \
                           ctx->tickets + TICKET_MARCH, ctx->flags, ctx->mip, ctx->box, ctx->slots, slot_cap)
-    const bool shared = ctx->tune.side_sms != 0;
+    const bool shared = ctx->tune.side_sms != 0 || n_rays > (uint32_t)num_sms() * SCHEDULERS * WARP;
     switch (cg.mode) {
         case COUNT_POW2:
             st = shared ? TN_COUNT(COUNT_POW2, COUNT_DEPTH_SHARED) : TN_COUNT(COUNT_POW2, COUNT_DEPTH);
