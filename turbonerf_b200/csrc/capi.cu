@@ -74,6 +74,10 @@ int num_sms() {
     return cached;
 }
 
+// Scratch grown to at least n elements, with nothing in it: every reader reads what its own call wrote. A
+// clear would go to the legacy stream, which does not order it before the call's kernels on a non-blocking
+// stream, and the allocation after it waits for it now and then: of five processes' median first marches on a
+// fresh context, 2^15 rays, the slowest took 1.95 ms with the clear and 0.92 without (0.90 and 0.87 the fastest).
 template <typename T>
 static int ensure(T*& ptr, size_t& cap, size_t n, const char* what) {
     if (n <= cap) return TN_OK;
@@ -83,7 +87,6 @@ static int ensure(T*& ptr, size_t& cap, size_t n, const char* what) {
     cudaError_t e = cudaMalloc(&fresh, want * sizeof(T));
     if (e != cudaSuccess) return fail(TN_E_CUDA, "%s: cudaMalloc(%zu) failed: %s (reserve scratch with tn_ctx_reserve "
                                       "before capturing a graph)", what, want * sizeof(T), cudaGetErrorString(e));
-    cudaMemset(fresh, 0, want * sizeof(T));
     if (ptr) cudaFree(ptr);
     ptr = fresh;
     cap = want;
@@ -94,7 +97,13 @@ int ensure_block_u32(tn_ctx* ctx, size_t n) { return ensure(ctx->block_u32, ctx-
 int ensure_block_f32(tn_ctx* ctx, size_t n) { return ensure(ctx->block_f32, ctx->block_f32_cap, n, "scratch(f32)"); }
 int ensure_mip(tn_ctx* ctx, size_t bytes) { return ensure(ctx->mip, ctx->mip_cap, bytes, "scratch(mip)"); }
 int ensure_slots(tn_ctx* ctx, size_t n) { return ensure(ctx->slots, ctx->slots_cap, n, "scratch(slots)"); }
-int ensure_render_ws(tn_ctx* ctx, size_t bytes) { return ensure(ctx->render_ws, ctx->render_ws_cap, bytes, "scratch(render)"); }
+// Zeroed when it grows, on the caller's stream: a network may compute on the sample slots past the live ones.
+int ensure_render_ws(tn_ctx* ctx, size_t bytes, cudaStream_t stream) {
+    const size_t before = ctx->render_ws_cap;
+    const int st = ensure(ctx->render_ws, ctx->render_ws_cap, bytes, "scratch(render)");
+    if (st != TN_OK || ctx->render_ws_cap == before) return st;
+    return cuda_status(cudaMemsetAsync(ctx->render_ws, 0, ctx->render_ws_cap, stream), "scratch(render)");
+}
 
 int validate_grid(const tn_grid_desc* grid) {
     TN_REQUIRE(grid != nullptr, TN_E_NULL, "grid descriptor is NULL");

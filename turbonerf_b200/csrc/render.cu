@@ -593,7 +593,7 @@ int tn_render(tn_ctx* ctx, tn_stream_t stream, const tn_render_desc* desc, const
     const size_t mip1_words = ((size_t)mip_blocks + 63) / 64 * 16;
     const size_t mip_words = mip1_words + ((size_t)mip2_blocks + 63) / 64 * 16;
     const size_t smp_words = (size_t)12 * cap;
-    st = ensure_render_ws(ctx, (ray_words + list_words + 16 + mip_words + smp_words) * 4);
+    st = ensure_render_ws(ctx, (ray_words + list_words + 16 + mip_words + smp_words) * 4, stream);
     if (st != TN_OK) return st;
     float* rays = reinterpret_cast<float*>(ctx->render_ws);
     float *ori = rays, *dir = rays + 3 * (size_t)n, *ray_t = rays + 6 * (size_t)n, *ray_tmax = rays + 7 * (size_t)n,

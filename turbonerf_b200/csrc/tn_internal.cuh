@@ -59,7 +59,7 @@ int ensure_block_f32(tn_ctx* ctx, size_t n);
 int ensure_mip(tn_ctx* ctx, size_t bytes);
 int ensure_slots(tn_ctx* ctx, size_t n);
 uint32_t slot_capacity(uint32_t n_rays, uint32_t max_steps);  // step-position slots per ray (march.cu)
-int ensure_render_ws(tn_ctx* ctx, size_t bytes);
+int ensure_render_ws(tn_ctx* ctx, size_t bytes, cudaStream_t stream);
 bool stream_capturing(cudaStream_t s);
 int num_sms();
 
