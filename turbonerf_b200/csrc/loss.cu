@@ -2359,9 +2359,7 @@ train_losses_kernel(Samples S, uint32_t n_rays, const uint32_t* n_dev, uint32_t 
     };
     auto slots_of = [&](uint32_t o, uint32_t n) { return n + (VEC ? (o & 3u) : 0u); };  // slots the ray takes
     uint32_t most = 0;  // slots of the longest ray left to several warps
-    for (uint32_t k = wid;; k += W) {
-        const uint32_t r = block_ray(k);
-        if (r >= n_live) break;
+    for (uint32_t r = block_ray(wid); r < n_live; r += gridDim.x * W) {  // block_ray(wid + i W)
         const uint32_t o = offsets[r], n = counts[r], span = slots_of(o, n);
         if (span <= RB_MAX)
             train_losses_ray_blocked<VEC, RB_SPL, false>(S, r, o, n, lane, min_t, inv_nrays, grad_scale, lam, target, bg,
