@@ -163,7 +163,9 @@ int tn_rays_init_bbox(tn_stream_t stream, uint32_t n_rays, uint32_t ray_stride, 
  * n_steps, and batch_info[2] = total samples of all n_rays rays. The offsets themselves are
  * written by tn_march_emit. batch_size is the sample capacity (reference batch_size);
  * batch_size = UINT32_MAX disables the cut (render use: every ray is kept and
- * batch_info = {n_rays, total, total}). */
+ * batch_info = {n_rays, total, total}). The bitfield has to be 16-byte aligned at resolutions 16 to
+ * 128 (TN_E_INVALID otherwise); at others it may start at any byte, and is read faster from a multiple
+ * of 4. Nothing of a call's grid stays in the context for the next. */
 int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, const uint8_t* bitfield,
                    const tn_bbox* bbox, const tn_march_desc* march, uint32_t n_rays, uint32_t ray_stride,
                    const uint32_t* n_rays_dev, const float* ori, const float* dir, const float* ray_t,
@@ -176,7 +178,10 @@ int tn_march_count(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, co
  * dir[3] (0.5*d+0.5), dt (= dt/aabb_size, the compositor's dt), m_norm, dt_norm and
  * img_id (optional, from ray_img_id). offsets holds the exclusive scan of n_steps for all
  * n_rays rays (rays at or beyond the cut emit nothing). Must follow tn_march_count on the
- * same context with the same n_rays: it expands the step positions that pass recorded. */
+ * same context with the same n_rays: it expands the step positions that pass recorded, and marches on
+ * for rays with more samples than that pass keeps. Where the bitfield has changed in between, that
+ * march stops once the ray is out of the box, or at max_iterations, and the samples it did not find
+ * are placed there. */
 int tn_march_emit(tn_ctx* ctx, tn_stream_t stream, const tn_grid_desc* grid, const uint8_t* bitfield,
                   const tn_bbox* bbox, const tn_march_desc* march, float inv_aabb_size, uint32_t n_rays,
                   uint32_t ray_stride, uint32_t sample_stride, const uint32_t* batch_info,

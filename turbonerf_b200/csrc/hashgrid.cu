@@ -233,8 +233,8 @@ hg_backward_kernel(HashLevels H, uint32_t n, const uint32_t* __restrict__ n_dev,
 // a short batch. A cell shared with the sample before, as along a ray, is that one's to list; bits already
 // set are seen with a plain read and skip their atomic; the two corners of an x edge have theirs in one word
 // for 31 of 32 x, read and set as one; a block's new entries take one counter atomic.
-// Bound by the L2's atomics with a result (about 17 G a second; one a new entry is what the edges halve) and
-// by random reads. The backward with its list, 2^18 samples of 16 levels along rays and uniform: 310 and
+// Bound by the atomics that return and the random reads of the bitmap before them (28 of 43 stall cycles an
+// issued instruction wait for them). The backward with its list, 2^18 samples of 16 levels along rays and uniform: 310 and
 // 485 us; 467 and 590 where one kernel added and listed a sample a thread, 416 and 609 with this kernel
 // one atomic a corner, lanes compared entry by entry and one counter atomic a warp. Listing inside
 // the runs of hg_backward_kernel, edges together: 375 and 424, but 8000 samples 30 and 28 where this takes 22 and 25.
